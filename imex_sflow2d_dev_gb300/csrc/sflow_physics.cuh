@@ -14,7 +14,7 @@
 #include <cfloat>
 #include <cstdint>
 
-#include "sflow_math.h"
+#include "sflow_pow.h"
 #include "sflow_types.cuh"
 
 namespace sflow {
@@ -30,11 +30,12 @@ template <class R>
 __device__ __forceinline__ R rmax(R a, R b) { return a > b ? a : b; }
 template <class R>
 __device__ __forceinline__ R sq(R a) { return a * a; }
-// x^y and log x: in the FP64 form the library's own functions (sflow_math.h),
+// x^y and log x: in the FP64 form the library's own functions (sflow_math.h;
+// x^y through its quick evaluation with the same bits, sflow_pow.h),
 // which give the oracle's bits; in the FP32 form CUDA's powf and logf.
 template <class R>
 __device__ __forceinline__ R rpow(R x, R y) {
-  if constexpr (sizeof(R) == 8) return sfm_pow(x, y);
+  if constexpr (sizeof(R) == 8) return sfm_pow_quick(x, y);
   else return powf(x, y);
 }
 template <class R>
