@@ -14,6 +14,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "sflow_div64.cuh"
 #include "sflow_pow.h"
 #include "sflow_types.cuh"
 
@@ -570,305 +571,21 @@ __device__ __forceinline__ void semi_impl_terms(const Phys<R>& P, const Geo<R>& 
 }
 
 // ---------------------------------------------------------------------------
-// Implicit friction (constitutive_2d.f90:3513-4009, rheology 1 and 6) with
-// the gas-density / temperature closure of c_phys_var (1154-1322), written
-// once over a number type N: double for the residual, Cplx for the
-// complex-step Jacobian of the plain FP64 form (solver_2d.f90:2302-2367,
-// the derivative the reference takes).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double dsqrt(double a) { return sqrt(a); }
-__device__ __forceinline__ double val(double a) { return a; }
-
-// Complex numbers of the complex-step Jacobian with the arithmetic written
-// out: textbook product, Smith's quotient (R. L. Smith, CACM 5(8), 1962),
-// principal square root sqrt((|z| + |x|)/2).  The oracle spells the same
-// formulas in C; compiled without contraction (--fmad=false), the two give
-// the same Jacobian bits, and so the same Newton iterates.  A real operand
-// is a complex number with zero imaginary part, for which each operation
-// returns the real result exactly.
-struct Cplx {
-  double re, im;
-  __device__ Cplx() {}
-  __device__ Cplx(double r) : re(r), im(0.0) {}
-  __device__ Cplx(double r, double i) : re(r), im(i) {}
-};
-__device__ __forceinline__ Cplx operator+(Cplx a, Cplx b) { return Cplx(a.re + b.re, a.im + b.im); }
-__device__ __forceinline__ Cplx operator-(Cplx a, Cplx b) { return Cplx(a.re - b.re, a.im - b.im); }
-__device__ __forceinline__ Cplx operator*(Cplx a, Cplx b) {
-  return Cplx(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re);
-}
-__device__ __forceinline__ Cplx operator/(Cplx a, Cplx b) {
-  if (fabs(b.re) >= fabs(b.im)) {
-    const double r = b.im / b.re, den = b.re + b.im * r;
-    return Cplx((a.re + a.im * r) / den, (a.im - a.re * r) / den);
-  }
-  const double r = b.re / b.im, den = b.re * r + b.im;
-  return Cplx((a.re * r + a.im) / den, (a.im * r - a.re) / den);
-}
-__device__ __forceinline__ Cplx dsqrt(Cplx z) {
-  const double ar = fabs(z.re), ai = fabs(z.im);
-  if (ar == 0.0 && ai == 0.0) return Cplx(0.0, z.im);
-  double m;
-  if (ai == 0.0) m = ar;
-  else if (ar == 0.0) m = ai;
-  else if (ar >= ai) { const double t = ai / ar; m = ar * sqrt(1.0 + t * t); }
-  else { const double t = ar / ai; m = ai * sqrt(1.0 + t * t); }
-  const double t = sqrt((ar + m) * 0.5);
-  if (z.re >= 0.0) return Cplx(t, z.im / (2.0 * t));
-  return Cplx(ai / (2.0 * t), copysign(t, z.im));
-}
-__device__ __forceinline__ double val(Cplx a) { return a.re; }
-
-template <class N, int NS>
-__device__ __forceinline__ void implicit_terms(const Phys<double>& P, double Bx, double By,
-                                               const N* q, N& nh1, N& nh2) {
-  nh1 = N(0.0);
-  nh2 = N(0.0);
-  if (!P.rheo) return;
-  constexpr int ns = NS;
-  // c_phys_var
-  N h, u, v, T, rho_m;
-  if (val(q[0]) > kEps) {
-    N inv_cqj1 = N(1.0) / q[0];
-    N xs_tot = N(0.0), dcp = N(0.0), dinv = N(0.0);
-    for (int i = 0; i < ns; ++i) {
-      N xs = q[4 + i] * inv_cqj1;
-      xs_tot = xs_tot + xs;
-    }
-    for (int i = 0; i < ns; ++i) {
-      N xs = q[4 + i] * inv_cqj1;
-      dcp = dcp + xs * N(P.sp_heat_s[i]);
-      dinv = dinv + xs * N(P.inv_rho_s[i]);
-    }
-    N xc = N(1.0) - xs_tot;
-    N cp_c = P.gas ? ((xc - N(0.0)) * N(P.sp_heat_a) + N(0.0)) / xc : N(P.sp_heat_l);
-    N cmix = dcp + xc * cp_c;
-    if (val(q[0]) > P.eps_sing_d) {
-      if (P.energy) T = (q[3] - N(0.5) * (q[1] * q[1] + q[2] * q[2]) * inv_cqj1) / (q[0] * cmix);
-      else T = q[3] / (q[0] * cmix);
-      if (val(T) <= 0.0) T = N(P.T_ambient);
-    } else {
-      T = N(P.T_ambient);
-    }
-    N inv_rho_c;
-    if (P.gas) {
-      N Rc = ((xc - N(0.0)) * N(P.sp_gas_const_a) + N(0.0)) / xc;
-      inv_rho_c = Rc * T * N(P.inv_pres);
-    } else {
-      inv_rho_c = N(P.inv_rho_l);
-    }
-    N inv_rhom = dinv + xc * inv_rho_c;
-    rho_m = N(1.0) / inv_rhom;
-    h = q[0] * inv_rhom;
-    if (val(q[0]) > P.eps_sing_d) {
-      u = q[1] * inv_cqj1;
-      v = q[2] * inv_cqj1;
-    } else {
-      N q4 = q[0] * q[0];
-      q4 = q4 * q4;
-      N den = dsqrt(q4 + N(P.eps_sing4));
-      u = N(P.sqrt2) * q[0] * q[1] / den;
-      v = N(P.sqrt2) * q[0] * q[2] / den;
-    }
-  } else {
-    return;  // h = u = v = 0: mod_vel = 0, no friction
-  }
-  N red_grav = (rho_m - N(P.rho_a_amb)) / rho_m * N(P.grav);
-  N w = P.slope_corr ? (u * N(Bx) + v * N(By)) : N(0.0);
-  N mod_vel2 = u * u + v * v + w * w;
-  N mod_vel = dsqrt(mod_vel2);
-  if (val(mod_vel) != 0.0) {
-    if (P.rheo_model == 1) {
-      N turb = rho_m * red_grav / N(P.xi) * mod_vel2;
-      nh1 = nh1 - turb * (u / mod_vel);
-      nh2 = nh2 - turb * (v / mod_vel);
-    } else if (P.rheo_model == 6) {
-      N mod_vel_hor = dsqrt(u * u + v * v);
-      nh1 = nh1 - rho_m * (u / mod_vel_hor) * N(P.friction_factor) * mod_vel2;
-      nh2 = nh2 - rho_m * (v / mod_vel_hor) * N(P.friction_factor) * mod_vel2;
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// solver_2d.f90:1662-1996 solve_rk_step, 2021-2226 lnsrch, 2245-2284 eval_f
-// (normalize_q = T, normalize_f = F, opt_search_NL = T; implicit set {hu,hv})
-// ---------------------------------------------------------------------------
-struct NewtonCtx {
-  const Phys<double>* P;
-  double dt, a_diag, Bx, By;
-  const double* q_old;
-  const double* Rj;
-};
-
-template <int NS>
-__device__ __forceinline__ void newton_eval_f(const NewtonCtx& c, const double* qj, double* f,
-                                              double& scal_f) {
-  constexpr int nv = 4 + NS;
-  double nh1, nh2;
-  implicit_terms<double, NS>(*c.P, c.Bx, c.By, qj, nh1, nh2);
-  double s = 0.0;
-  for (int i = 0; i < nv; ++i) {
-    double nh = (i == 1) ? nh1 : (i == 2) ? nh2 : 0.0;
-    double Rj = c.Rj[i] - c.a_diag * nh;
-    f[i] = qj[i] - c.q_old[i] + c.dt * Rj;
-  }
-  for (int i = 0; i < nv; ++i) s += f[i] * f[i];
-  scal_f = 0.5 * s;
-}
-
-// Jacobian of f with respect to qj_rel for the implicit columns 1, 2
-// (solver_2d.f90:2302-2367): J(k,i) = qj_org_i delta_ki - dt a_diag
-// Im(NH_k(qj_rel qj_org + i h e_i qj_org)) / h with h = n_vars EPSILON, the
-// complex step of the reference, evaluated at qj_rel * qj_org.
-template <int NS>
-__device__ __forceinline__ void newton_jacobian(const NewtonCtx& c, const double* qj_rel,
-                                                const double* qj_org, double& s11, double& s12,
-                                                double& s21, double& s22) {
-  constexpr int nv = 4 + NS;
-  const double h = nv * kEps, one_by_h = 1.0 / h;
-  double jc[2][2];
-  for (int col = 1; col <= 2; ++col) {
-    Cplx qc[kMaxVars];
-    for (int k = 0; k < nv; ++k) qc[k] = Cplx(qj_rel[k] * qj_org[k]);
-    qc[col] = Cplx(qj_rel[col], h) * Cplx(qj_org[col]);
-    Cplx n1, n2;
-    implicit_terms<Cplx, NS>(*c.P, c.Bx, c.By, qc, n1, n2);
-    jc[0][col - 1] = 1.0 * n1.im * one_by_h;
-    jc[1][col - 1] = 1.0 * n2.im * one_by_h;
-  }
-  s11 = 1.0 * qj_org[1] - c.dt * c.a_diag * jc[0][0];
-  s12 = 0.0 - c.dt * c.a_diag * jc[0][1];
-  s21 = 0.0 - c.dt * c.a_diag * jc[1][0];
-  s22 = 1.0 * qj_org[2] - c.dt * c.a_diag * jc[1][1];
-}
-
-// returns iterations used (kMaxNewton+1 when the limit was reached)
-template <int NS>
-__device__ int solve_rk_step(const NewtonCtx& c, double* qj) {
-  constexpr int nv = 4 + NS;
-  const double STPMX = 100.0, TOLF = 1.0e-10, TOLMIN = 1.0e-6, TOLX = kEps;
-  double qj_org[kMaxVars], qj_rel[kMaxVars], f[kMaxVars], p[kMaxVars], g[kMaxVars],
-      x_old[kMaxVars], qt[kMaxVars];
-  double scal_f, scal_f_old;
-  bool check = false;
-  for (int i = 0; i < nv; ++i) {
-    g[i] = 0.0;
-    qj_org[i] = rmax(fabs(qj[i]), 1.0e-3);
-    qj_rel[i] = qj[i] / qj_org[i];
-  }
-  for (int it = 1; it <= kMaxNewton; ++it) {
-    newton_eval_f<NS>(c, qj, f, scal_f);
-    double mf = 0.0;
-    for (int i = 0; i < nv; ++i) mf = rmax(mf, fabs(f[i]));
-    if (mf < TOLF) return it;
-    if (!isfinite(scal_f)) return kMaxNewton + 1;   // NaN/Inf state: give up at once
-    double s11, s12, s21, s22;
-    newton_jacobian<NS>(c, qj_rel, qj_org, s11, s12, s21, s22);
-    // explicit rows: diagonal qj_org (mask11); coupling mask21 is zero
-    for (int i = 0; i < nv; ++i) p[i] = (i == 1 || i == 2) ? 0.0 : -(f[i] / qj_org[i]) + 0.0;
-    double d2a = f[1], d2b = f[2];
-    for (int i = 0; i < nv; ++i) {
-      if (i == 1 || i == 2) continue;
-      d2a = d2a - (f[i] / qj_org[i]) * 0.0;
-      d2b = d2b - (f[i] / qj_org[i]) * 0.0;
-    }
-    double inv_det = 1.0 / (s11 * s22 - s21 * s12);
-    p[1] = -((d2a * s22 - d2b * s12) * inv_det) + 0.0;
-    p[2] = -((s11 * d2b - s21 * d2a) * inv_det) + 0.0;
-    for (int i = 0; i < nv; ++i) x_old[i] = qj_rel[i];
-    scal_f_old = scal_f;
-    if (it > 1) {
-      double nr = 0.0;
-      for (int i = 0; i < nv; ++i) nr += qj_rel[i] * qj_rel[i];
-      double stpmax = STPMX * rmax(sqrt(nr), double(nv));
-      // grad_f = right_term . left_matrix: explicit columns diag qj_org
-      for (int i = 0; i < nv; ++i) g[i] = (i == 1 || i == 2) ? 0.0 : f[i] * qj_org[i];
-      g[1] = f[1] * s11 + f[2] * s21;
-      g[2] = f[1] * s12 + f[2] * s22;
-      // lnsrch
-      check = false;
-      double nrm = 0.0;
-      for (int i = 0; i < nv; ++i) nrm += p[i] * p[i];
-      nrm = sqrt(nrm);
-      if (nrm > stpmax)
-        for (int i = 0; i < nv; ++i) p[i] = p[i] * stpmax / nrm;
-      double slope = 0.0;
-      for (int i = 0; i < nv; ++i) slope += g[i] * p[i];
-      double mx = 0.0;
-      for (int i = 0; i < nv; ++i) {
-        double t = fabs(p[i]) / rmax(fabs(x_old[i]), 1.0);
-        if (i == 0 || t > mx) mx = t;
-      }
-      double alamin = TOLX / mx;
-      if (alamin == 0.0) {
-        for (int i = 0; i < nv; ++i) qj_rel[i] = x_old[i];
-      } else {
-        double alam = 1.0, alam2 = 0.0, f2 = 0.0, tmplam = 0.0;
-        for (int ls = 0; ls < 4096; ++ls) {
-          for (int i = 0; i < nv; ++i) {
-            qj_rel[i] = x_old[i] + alam * p[i];
-            qt[i] = qj_rel[i] * qj_org[i];
-          }
-          newton_eval_f<NS>(c, qt, f, scal_f);
-          if (scal_f <= 0.9 * scal_f_old) break;
-          if (alam < alamin) {
-            for (int i = 0; i < nv; ++i) qj_rel[i] = x_old[i];
-            scal_f = scal_f_old;
-            check = true;
-            break;
-          }
-          if (alam == 1.0) {
-            tmplam = -slope / (2.0 * (scal_f - scal_f_old - slope));
-          } else {
-            double rhs1 = scal_f - scal_f_old - alam * slope;
-            double rhs2 = f2 - scal_f_old - alam2 * slope;
-            double a = (rhs1 / sq(alam) - rhs2 / sq(alam2)) / (alam - alam2);
-            double b = (-alam2 * rhs1 / sq(alam) + alam * rhs2 / sq(alam2)) / (alam - alam2);
-            if (a == 0.0) {
-              tmplam = -slope / (2.0 * b);
-            } else {
-              double disc = b * b - 3.0 * a * slope;
-              if (disc < 0.0) tmplam = 0.5 * alam;
-              else if (b <= 0.0) tmplam = (-b + sqrt(disc)) / (3.0 * a);
-              else tmplam = -slope / (b + sqrt(disc));
-            }
-            if (tmplam > 0.5 * alam) tmplam = 0.5 * alam;
-          }
-          alam2 = alam;
-          f2 = scal_f;
-          alam = rmax(tmplam, 0.5 * alam);
-        }
-      }
-    } else {
-      for (int i = 0; i < nv; ++i) {
-        qj_rel[i] = x_old[i] + p[i];
-        qj[i] = qj_rel[i] * qj_org[i];
-      }
-      newton_eval_f<NS>(c, qj, f, scal_f);
-    }
-    for (int i = 0; i < nv; ++i) qj[i] = qj_rel[i] * qj_org[i];
-    mf = 0.0;
-    for (int i = 0; i < nv; ++i) mf = rmax(mf, fabs(f[i]));
-    if (mf < TOLF) return it;
-    if (check) {
-      double mc = 0.0;
-      for (int i = 0; i < nv; ++i)
-        mc = rmax(mc, fabs(g[i]) * rmax(fabs(qj_rel[i]), 1.0) / rmax(scal_f, 0.5 * nv));
-      check = mc < TOLMIN;
-    }
-    double mx = 0.0;
-    for (int i = 0; i < nv; ++i) mx = rmax(mx, fabs(qj_rel[i] - x_old[i]) / rmax(fabs(qj_rel[i]), 1.0));
-    if (mx < TOLX) return it;
-  }
-  return kMaxNewton + 1;
-}
-
-// ---------------------------------------------------------------------------
 // constitutive_2d.f90:5326-5404 settling_velocity and 4574-5153
 // eval_mass_exchange_terms (settling, erosion of the erodible layer, air
 // entrainment; no pore pressure / vaporisation)
 // ---------------------------------------------------------------------------
+// d / s < tol for d >= 0, s > 0: with the product unless the two lie within a
+// few units in the last place (the quotient then decides)
+template <class R>
+__device__ __forceinline__ bool rel_below(R d, R s, R tol) {
+  if constexpr (sizeof(R) == 8) {
+    const long long diff = d64_bits(d) - d64_bits(s * tol);
+    if (diff > 8 || diff < -8) return diff < 0;
+  }
+  return d / s < tol;
+}
+
 template <class R>
 __device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos, R rhoc,
                                                R inv_kin_visc) {
@@ -886,7 +603,7 @@ __device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos,
       else
         inv_sqrt_C_D = sqrt(Rey / (cst<R>(24.0) * (R(1) + cst<R>(0.15) * rpow<R>(Rey, cst<R>(0.687)))));
       sv = const_part * inv_sqrt_C_D;
-      if (fabs(sv_old - sv) / sv_old < cst<R>(1.0e-6)) return sv;
+      if (rel_below<R>(fabs(sv_old - sv), sv_old, cst<R>(1.0e-6))) return sv;
       Rey = diam * sv * inv_kin_visc;
     }
   }
