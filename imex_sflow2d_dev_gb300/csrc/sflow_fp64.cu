@@ -18,7 +18,7 @@ __global__ void k_eval_math(int which, long long n, const double* x, const doubl
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     double r;
     switch (which) {
-      case 0: r = sfm_pow_quick(x[i], y[i]); break;
+      case 0: r = sfm_pow_int(x[i], y[i]); break;
       case 1: r = sfm_log(x[i]); break;
       case 2: r = sfm_cos(x[i]); break;
       case 3: r = pow(x[i], y[i]); break;

@@ -600,8 +600,8 @@ __device__ __noinline__ void recon_side_edge(const KArgs<R>& a, const R* sqp, co
   for (int m = 0; m < 2; ++m) {
     const int i = nv + m;
     const R v1 = cell[i];
-    const R ul = (lo[0] <= R(0)) ? R(0) : lo[1 + m] / lo[0];
-    const R uh = (hi[0] <= R(0)) ? R(0) : hi[1 + m] / hi[0];
+    const R ul = (lo[0] <= R(0)) ? R(0) : rdiv<R>(lo[1 + m], lo[0]);
+    const R uh = (hi[0] <= R(0)) ? R(0) : rdiv<R>(hi[1 + m], hi[0]);
     R v0, v2;
     if (b0) { v0 = ul; v2 = QP(i, 1); }
     else if (b1) { v0 = QP(i, -1); v2 = uh; }
@@ -738,9 +738,10 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
   } else {
     const R den = a2 - a1;
     if constexpr (sizeof(R) == 8) {
-      const R fac = (a2 * a1) / den;
+      const Div64 vd = div64(den);
+      const R fac = quot64(a2 * a1, vd);
 #pragma unroll
-      for (int i = 0; i < nv; ++i) H[i] = (a2 * L.f[i] - a1 * Rt.f[i]) / den + fac * (Rt.q[i] - L.q[i]);
+      for (int i = 0; i < nv; ++i) H[i] = quot64(a2 * L.f[i] - a1 * Rt.f[i], vd) + fac * (Rt.q[i] - L.q[i]);
     } else {
       const R inv_den = fdiv(R(1), den);
       const R fac = (a2 * a1) * inv_den;
@@ -759,21 +760,28 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
         s2 = s2 * inv0;
       } else {
 #pragma unroll
-        for (int i = 0; i < ns; ++i) { s += H[4 + i] / H[0]; s2 += H[4 + i]; }
-        s2 = s2 / H[0];
+        for (int i = 0; i < ns; ++i) s2 += H[4 + i];
+        // s2 / H[0] >= 1 without the quotient: rounded, it reaches 1 exactly
+        // when s2 reaches H[0] (the next number below lies more than 2^-54 away)
+        const bool over = H[0] > R(0) ? s2 >= H[0] : (H[0] < R(0) ? s2 <= H[0] : s2 / H[0] >= R(1));
+        s2 = over ? R(1) : R(0);
+        if (over) {
+#pragma unroll
+          for (int i = 0; i < ns; ++i) s += rdiv<R>(H[4 + i], H[0]);
+        }
       }
       if (s2 >= R(1)) {
 #pragma unroll
-        for (int i = 0; i < ns; ++i) H[4 + i] = H[4 + i] / s;
+        for (int i = 0; i < ns; ++i) H[4 + i] = rdiv<R>(H[4 + i], s);
       }
     } else {
       R s = R(0);
 #pragma unroll
       for (int i = 0; i < ns; ++i) s += H[4 + i];
-      if (s / H[0] > R(1)) {
-        const R r = s / H[0];
+      const R r = rdiv<R>(s, H[0]);
+      if (r > R(1)) {
 #pragma unroll
-        for (int i = 0; i < ns; ++i) H[4 + i] = H[4 + i] / r;
+        for (int i = 0; i < ns; ++i) H[4 + i] = rdiv<R>(H[4 + i], r);
       }
     }
   }
@@ -1076,8 +1084,8 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
         R ax = rmax(sAx[cy * (TX + 1) + cx], sAx[cy * (TX + 1) + cx + 1]);
         R ay = (g.ny > 1) ? rmax(sAy[cy * TX + cx], sAy[(cy + 1) * TX + cx]) : R(0);
         if constexpr (sizeof(R) == 8) {
-          double dtx = (ax > 0.0) ? g.cfl * g.dx / ax : 1.0e300;
-          double dty = (ay > 0.0) ? g.cfl * g.dy / ay : 1.0e300;
+          double dtx = (ax > 0.0) ? ddiv64(g.cfl * g.dx, ax) : 1.0e300;
+          double dty = (ay > 0.0) ? ddiv64(g.cfl * g.dy, ay) : 1.0e300;
           dtloc = rmin(dtx, dty);
         } else {
           float dtx = (ax > 0.0f) ? fdiv(g.cfl_dx, ax) : 3.0e38f;
@@ -1301,7 +1309,7 @@ __device__ __forceinline__ unsigned assemble_fixes(const Phys<R>& P, R* q, CellQ
     if (ssum > q[0]) {
       if (cq) cq->valid = false;
       bool small;
-      if constexpr (sizeof(R) == 8) small = ((ssum - q[0]) / q[0] < 1.0e-10) || (q[0] < P.thr_eps);
+      if constexpr (sizeof(R) == 8) small = (rdiv<R>(ssum - q[0], q[0]) < 1.0e-10) || (q[0] < P.thr_eps);
       else small = !((ssum - q[0]) / q[0] > P.thr_1em10) || (q[0] < P.thr_eps);
       if (!small) st |= SFLOW_S_SOLID_GT_MASS;
       R s = R(0);
@@ -1536,7 +1544,7 @@ __device__ __forceinline__ void post_step_maps(const KArgs<R>& a, int64_t c, con
     R hm = a.hmax[c];
     a.hmax[c] = rmax(hm, qp[0]);
     if (qp[0] > a.pr.thr_1em3) {
-      R mv = sqrt(sq(qp[nv]) + sq(qp[nv + 1]));
+      R mv = rroot<R>(sq(qp[nv]) + sq(qp[nv + 1]));
       a.pdynmax[c] = rmax(a.pdynmax[c], p_dyn);
       a.mvmax[c] = rmax(a.mvmax[c], mv);
     }
@@ -1569,6 +1577,7 @@ __device__ __forceinline__ unsigned stage_cell(const KArgs<R>& a, const Geo<R>& 
 #pragma unroll
     for (int i = 0; i < nv; ++i) { si[i] = 0.0; qsi[i] = qfv[i]; qg[i] = qfv[i]; }
     if (a_diag != 0.0) {
+      const Div64 vdta = div64(dt * a_diag);
       if (qfv[0] > 0.0) {
         qc_to_qp<double, NS>(P, qfv, qp);
         semi_impl_terms<double, NS>(P, geo, qp, si);
@@ -1579,12 +1588,13 @@ __device__ __forceinline__ unsigned stage_cell(const KArgs<R>& a, const Geo<R>& 
         } else if (qsi[1] * qfv[1] < 0.0 || qsi[2] * qfv[2] < 0.0) {
           qsi[1] = 0.0; qsi[2] = 0.0;
         } else {
-          double m1 = sqrt(sq(qsi[1]) + sq(qsi[2])), m0 = sqrt(sq(qfv[1]) + sq(qfv[2]));
-          qsi[1] = m1 * qfv[1] / m0;
-          qsi[2] = m1 * qfv[2] / m0;
+          const double m1 = dsqrt64(sq(qsi[1]) + sq(qsi[2]));
+          const Div64 m0 = div64(dsqrt64(sq(qfv[1]) + sq(qfv[2])));
+          qsi[1] = quot64(m1 * qfv[1], m0);
+          qsi[2] = quot64(m1 * qfv[2], m0);
         }
 #pragma unroll
-        for (int i = 0; i < nv; ++i) { si[i] = (qsi[i] - qfv[i]) / (dt * a_diag); qg[i] = qsi[i]; }
+        for (int i = 0; i < nv; ++i) { si[i] = quot64(qsi[i] - qfv[i], vdta); qg[i] = qsi[i]; }
 #pragma unroll
         for (int i = 0; i < nv; ++i) Rj[i] = (s1[i] - s2[i]) - a_diag * si[i];
         NewtonCtx nc{&P, dt, a_diag, geo.Bx, geo.By, q0, Rj};
@@ -1596,13 +1606,14 @@ __device__ __forceinline__ unsigned stage_cell(const KArgs<R>& a, const Geo<R>& 
         } else if (qg[1] * qsi[1] <= 0.0 && qg[2] * qsi[2] <= 0.0) {
           qg[1] = 0.0; qg[2] = 0.0;
         } else {
-          double m1 = sqrt(sq(qg[1]) + sq(qg[2])), m0 = sqrt(sq(qsi[1]) + sq(qsi[2]));
-          qg[1] = m1 * qsi[1] / m0;
-          qg[2] = m1 * qsi[2] / m0;
+          const double m1 = dsqrt64(sq(qg[1]) + sq(qg[2]));
+          const Div64 m0 = div64(dsqrt64(sq(qsi[1]) + sq(qsi[2])));
+          qg[1] = quot64(m1 * qsi[1], m0);
+          qg[2] = quot64(m1 * qsi[2], m0);
         }
       }
 #pragma unroll
-      for (int i = 0; i < nv; ++i) rn_out[i] = (qg[i] - qsi[i]) / (dt * a_diag) + si[i];
+      for (int i = 0; i < nv; ++i) rn_out[i] = quot64(qg[i] - qsi[i], vdta) + si[i];
     } else {
 #pragma unroll
       for (int i = 0; i < nv; ++i) rn_out[i] = 0.0;

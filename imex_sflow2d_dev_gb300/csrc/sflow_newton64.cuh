@@ -12,8 +12,8 @@
 // left out or shared does not change them:
 //  * only the columns hu and hv are perturbed, so q(1), q(4) and the solid
 //    masses, and every quantity formed from them alone, stay real;
-//  * the quotients by one divisor share its reciprocal (sflow_div64.cuh);
-//    the real divisors of the two columns equal those of the real
+//  * divisions and square roots run on the integer pipes, and the quotients
+//    by one divisor share its reciprocal (sflow_div64.cuh); the real divisors of the two columns equal those of the real
 //    evaluation unless a perturbation reaches them (tested on the bits);
 //  * the end-of-iteration residual is that of the next iteration's start;
 //  * the line search's slope, step bound and least step are formed only
@@ -42,7 +42,7 @@ struct Cplx {
 // a / b by Smith's quotient; v: the divisor b.re with its reciprocal when
 // |b.re| >= |b.im|.  known / quot: a numerator real part whose quotient by
 // v.d is already at hand.
-__device__ __forceinline__ Cplx cdiv_plain(Cplx a, Cplx b) {
+static __device__ __noinline__ Cplx cdiv_plain(Cplx a, Cplx b) {
   if (!d64_lt(fabs(b.re), fabs(b.im))) {
     const double r = b.im / b.re, den = b.re + b.im * r;
     return Cplx{(a.re + a.im * r) / den, (a.im - a.re * r) / den};
@@ -92,7 +92,8 @@ struct FrictPoint {
   double s0;              // film: sqrt2 q(1)
   Div64 den;              // film: sqrt(q(1)^4 + eps_sing^4)
   double dinv;            // sum x_s / rho_s
-  Div64 dinvr;            // 1/rho_m (its reciprocal is rho_m)
+  Div64 dinvr;            // 1/rho_m
+  double rho;             // rho_m
   Div64 drho;             // rho_m
   double nrg, qrg, rg;    // rho_m - rho_a, (rho_m - rho_a)/rho_m, reduced gravity
   double u, v, w, m2, mod;
@@ -110,7 +111,7 @@ __device__ __forceinline__ void friction_real(const Phys<double>& P, double Bx, 
   f.live = P.rheo && d64_gt_pos(q[0], kEps);
   if (!f.live) return;
   f.film = !d64_gt_pos(q[0], P.eps_sing_d);
-  f.inv = 1.0 / q[0];
+  f.inv = ddiv64(1.0, q[0]);
   double xs_tot = 0.0, dcp = 0.0, dinv = 0.0;
 #pragma unroll
   for (int i = 0; i < ns; ++i) {
@@ -124,31 +125,32 @@ __device__ __forceinline__ void friction_real(const Phys<double>& P, double Bx, 
   f.t_amb = f.film;
   double inv_rho_c;
   if (P.gas) {
+    const Div64 dxc = div64(f.xc);
     double T;
     if (!f.film) {
-      const double cp_c = (f.xc * P.sp_heat_a + 0.0) / f.xc;
+      const double cp_c = quot64(f.xc * P.sp_heat_a + 0.0, dxc);
       const double cmix = dcp + f.xc * cp_c;
       const double e = P.energy ? q[3] - 0.5 * (q[1] * q[1] + q[2] * q[2]) * f.inv : q[3];
       if (P.energy) {
         f.dT = div64(q[0] * cmix);
         T = quot64(e, f.dT);
       } else {
-        T = e / (q[0] * cmix);
+        T = ddiv64(e, q[0] * cmix);
       }
       f.t_amb = T <= 0.0;
     }
     if (f.t_amb) T = P.T_ambient;
-    f.Rc = (f.xc * P.sp_gas_const_a + 0.0) / f.xc;
+    f.Rc = quot64(f.xc * P.sp_gas_const_a + 0.0, dxc);
     inv_rho_c = f.Rc * T * P.inv_pres;
   } else {
     inv_rho_c = P.inv_rho_l;   // the temperature does not enter
   }
   f.dinvr = div64(dinv + f.xc * inv_rho_c);
-  const double rho_m = f.dinvr.zh;
+  const double rho_m = f.rho = quot64(1.0, f.dinvr);
   if (f.film) {
     double q4 = q[0] * q[0];
     q4 = q4 * q4;
-    f.den = div64(sqrt(q4 + P.eps_sing4));
+    f.den = div64(dsqrt64(q4 + P.eps_sing4));
     f.s0 = P.sqrt2 * q[0];
     f.u = quot64(f.s0 * q[1], f.den);
     f.v = quot64(f.s0 * q[2], f.den);
@@ -162,7 +164,7 @@ __device__ __forceinline__ void friction_real(const Phys<double>& P, double Bx, 
   f.rg = f.qrg * P.grav;
   f.w = P.slope_corr ? (f.u * Bx + f.v * By) : 0.0;
   f.m2 = f.u * f.u + f.v * f.v + f.w * f.w;
-  f.mod = sqrt(f.m2);
+  f.mod = dsqrt64(f.m2);
   if (!d64_zero(f.mod)) {
     f.dmod = div64(f.mod);
     f.um = quot64(f.u, f.dmod);
@@ -191,7 +193,7 @@ __device__ __forceinline__ void friction_imag(const Phys<double>& P, double Bx, 
   const Cplx a = (COL == 0) ? Cplx{q1, e} : Cplx{q1, 0.0};
   const Cplx b = (COL == 1) ? Cplx{q2, e} : Cplx{q2, 0.0};
   // mixture density and reduced gravity: complex through the temperature
-  Cplx rho{f.dinvr.zh, 0.0}, rg{f.rg, 0.0};
+  Cplx rho{f.rho, 0.0}, rg{f.rg, 0.0};
   if (P.gas && P.energy && !f.film) {
     const double pr = (COL == 0) ? q1 : q2;
     const double two = pr * e + e * pr;
@@ -202,10 +204,10 @@ __device__ __forceinline__ void friction_imag(const Phys<double>& P, double Bx, 
     if (!(Tre <= 0.0)) {
       const double Tim = quot64(nim, f.dT);
       const Cplx ir{f.dinv + f.xc * (f.Rc * Tre * P.inv_pres), f.xc * (f.Rc * Tim * P.inv_pres)};
-      rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.dinvr.zh);
+      rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.rho);
     } else {
       const Cplx ir{f.dinv + f.xc * (f.Rc * P.T_ambient * P.inv_pres), 0.0};
-      rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.dinvr.zh);
+      rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.rho);
     }
     const Cplx qr = cdiv(Cplx{rho.re - P.rho_a_amb, rho.im}, rho, f.drho, f.nrg, f.qrg);
     rg = Cplx{qr.re * P.grav, qr.im * P.grav};
@@ -291,7 +293,7 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
 #pragma unroll
   for (int i = 0; i < nv; ++i) {
     org[i] = d64_lt(1.0e-3, fabs(qj[i])) ? fabs(qj[i]) : 1.0e-3;
-    rel[i] = qj[i] / org[i];
+    rel[i] = ddiv64(qj[i], org[i]);
     xo[i] = rel[i] * org[i];
     same = same && d64_bits(xo[i]) == d64_bits(qj[i]);
   }
@@ -309,11 +311,11 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
     friction_imag<1>(P, c.Bx, c.By, dxi, fp, qj[1], qj[2], qj[3], h * org[2], j12, j22);
     const double s11 = org[1] - dta * (j11 * one_by_h), s12 = 0.0 - dta * (j12 * one_by_h);
     const double s21 = 0.0 - dta * (j21 * one_by_h), s22 = org[2] - dta * (j22 * one_by_h);
-    const double inv_det = 1.0 / (s11 * s22 - s21 * s12);
+    const double inv_det = ddiv64(1.0, s11 * s22 - s21 * s12);
 #pragma unroll
     for (int i = 0; i < nv; ++i) {
       // explicit rows: diagonal org, no coupling into the implicit rows
-      if (i != 1 && i != 2) p[i] = d64_zero(f[i]) ? 0.0 : -(f[i] / org[i]);
+      if (i != 1 && i != 2) p[i] = d64_zero(f[i]) ? 0.0 : -ddiv64(f[i], org[i]);
       xo[i] = rel[i];
     }
     p[1] = -((f[1] * s22 - f[2] * s12) * inv_det) + 0.0;

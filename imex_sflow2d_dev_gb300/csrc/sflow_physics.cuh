@@ -32,11 +32,11 @@ __device__ __forceinline__ R rmax(R a, R b) { return a > b ? a : b; }
 template <class R>
 __device__ __forceinline__ R sq(R a) { return a * a; }
 // x^y and log x: in the FP64 form the library's own functions (sflow_math.h;
-// x^y through its quick evaluation with the same bits, sflow_pow.h),
+// x^y on the integer pipes with the same bits, sflow_pow.h),
 // which give the oracle's bits; in the FP32 form CUDA's powf and logf.
 template <class R>
 __device__ __forceinline__ R rpow(R x, R y) {
-  if constexpr (sizeof(R) == 8) return sfm_pow_quick(x, y);
+  if constexpr (sizeof(R) == 8) return sfm_pow_int(x, y);
   else return powf(x, y);
 }
 template <class R>
@@ -51,7 +51,38 @@ __device__ __forceinline__ R rlog(R x) {
 template <class R>
 __device__ __forceinline__ R fdiv(R a, R b) {
   if constexpr (sizeof(R) == 4) return __fdividef(a, b);
+  else return ddiv64(a, b);
+}
+// a / b and sqrt(x): the FP64 form's on the integer pipes with the same bits
+// (sflow_div64.cuh), the FP32 form's as the compiler makes them.
+template <class R>
+__device__ __forceinline__ R rdiv(R a, R b) {
+  if constexpr (sizeof(R) == 8) return ddiv64(a, b);
   else return a / b;
+}
+template <class R>
+__device__ __forceinline__ R rroot(R x) {
+  if constexpr (sizeof(R) == 8) return dsqrt64(x);
+  else return sqrt(x);
+}
+// a divisor that several quotients share
+template <class R>
+struct Divisor {
+  R d;
+};
+template <>
+struct Divisor<double> {
+  Div64 v;
+};
+template <class R>
+__device__ __forceinline__ Divisor<R> divisor(R d) {
+  if constexpr (sizeof(R) == 8) return Divisor<R>{div64(d)};
+  else return Divisor<R>{d};
+}
+template <class R>
+__device__ __forceinline__ R quotient(R a, const Divisor<R>& v) {
+  if constexpr (sizeof(R) == 8) return quot64(a, v.v);
+  else return a / v.d;
 }
 
 // ---------------------------------------------------------------------------
@@ -101,28 +132,28 @@ template <class R>
 __device__ __forceinline__ R minmod(R a, R b) {
   R aa = fabs(a), ab = fabs(b);
   if (rmin(aa, ab) <= R(0)) return R(0);
-  R sa = a / aa, sb = b / ab;
+  R sa = rdiv<R>(a, aa), sb = rdiv<R>(b, ab);
   return cst<R>(0.5) * (sa + sb) * rmin(aa, ab);
 }
 template <class R>
 __device__ __forceinline__ R maxmod(R a, R b) {
   if (fabs(a * b) <= R(0)) return R(0);
-  R sa = a / fabs(a), sb = b / fabs(b);
+  R sa = rdiv<R>(a, fabs(a)), sb = rdiv<R>(b, fabs(b));
   return cst<R>(0.5) * (sa + sb) * rmax(fabs(a), fabs(b));
 }
 // LIM >= 0: the limiter of every variable, known at compile time; -1: lim
 template <class R, int LIM = -1>
 __device__ __forceinline__ R limit(R v0, R v1, R v2, R z0, R z1, R z2, int lim, R theta) {
-  R a = (v2 - v1) / (z2 - z1);
-  R b = (v1 - v0) / (z1 - z0);
+  R a = rdiv<R>(v2 - v1, z2 - z1);
+  R b = rdiv<R>(v1 - v0, z1 - z0);
   if constexpr (LIM >= 0) lim = LIM;
   switch (lim) {
     case 0: return R(0);
     case 1: return minmod(a, b);
     case 2: return maxmod(minmod(a, cst<R>(2.0) * b), minmod(cst<R>(2.0) * a, b));
-    case 3: { R c = (v2 - v0) / (z2 - z0); return minmod(c, theta * minmod(a, b)); }
-    case 4: { R c = (v2 - v0) / (z2 - z0); return minmod(c, cst<R>(2.0) * minmod(a, b)); }
-    case 5: return (v2 - v0) / (z2 - z0);
+    case 3: { R c = rdiv<R>(v2 - v0, z2 - z0); return minmod(c, theta * minmod(a, b)); }
+    case 4: { R c = rdiv<R>(v2 - v0, z2 - z0); return minmod(c, cst<R>(2.0) * minmod(a, b)); }
+    case 5: return rdiv<R>(v2 - v0, z2 - z0);
     case 6: return a;
     case 7: return b;
   }
@@ -173,7 +204,7 @@ __device__ __forceinline__ R qc_to_qp(const Phys<R>& P, const R* q, R* qp) {
     // as such; the FP64 form keeps the reference's operations)
     R Rc;
     if constexpr (sizeof(R) == 4) Rc = P.sp_gas_const_a;
-    else Rc = (xc > P.thr_eps) ? ((xc - R(0)) * P.sp_gas_const_a + R(0)) / xc : P.sp_gas_const_a;
+    else Rc = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_gas_const_a + R(0), xc) : P.sp_gas_const_a;
     inv_rho_c = Rc * T * P.inv_pres;
   } else {
     inv_rho_c = P.inv_rho_l;
@@ -190,9 +221,9 @@ __device__ __forceinline__ R qc_to_qp(const Phys<R>& P, const R* q, R* qp) {
   } else {
     if constexpr (sizeof(R) == 8) {
       R q12 = q[0] * q[0];
-      R den = sqrt(q12 * q12 + P.eps_sing4);
-      u = P.sqrt2 * q[0] * q[1] / den;
-      v = P.sqrt2 * q[0] * q[2] / den;
+      const Divisor<R> den = divisor<R>(rroot<R>(q12 * q12 + P.eps_sing4));
+      u = quotient<R>(P.sqrt2 * q[0] * q[1], den);
+      v = quotient<R>(P.sqrt2 * q[0] * q[2], den);
     } else {
       // same expression scaled by eps_sing: q1^4 and eps_sing^4 (1e-40)
       // are below the float range, (q1/eps)^4 is not
@@ -237,7 +268,7 @@ __device__ __forceinline__ void qp_to_qc(const Phys<R>& P, const R* qp, R* qc) {
     R rho_a = fdiv(P.pres, P.sp_gas_const_a * r_T);
     // carrier of air alone: ((1 - at) rho_a) / (1 - at) is rho_a
     if constexpr (sizeof(R) == 4) rho_c = rho_a;
-    else rho_c = ((R(1) - R(0) - at - R(0)) * rho_a + R(0)) / (R(1) - R(0) - at);
+    else rho_c = rdiv<R>((R(1) - R(0) - at - R(0)) * rho_a + R(0), R(1) - R(0) - at);
   } else {
     rho_c = P.rho_l;
   }
@@ -250,7 +281,7 @@ __device__ __forceinline__ void qp_to_qc(const Phys<R>& P, const R* qp, R* qc) {
   R cp_c;
   if (P.gas) {
     if constexpr (sizeof(R) == 4) cp_c = P.sp_heat_a;   // (x_c c_a) / x_c
-    else cp_c = (xc > P.thr_eps) ? ((xc - R(0)) * P.sp_heat_a + R(0)) / xc : P.sp_heat_a;
+    else cp_c = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_heat_a + R(0), xc) : P.sp_heat_a;
   } else {
     cp_c = P.sp_heat_l;
   }
@@ -295,17 +326,22 @@ __device__ __forceinline__ Mixt<R> mixt_var(const Phys<R>& P, const R* qpj, bool
     R rho_a = fdiv(P.pres, P.sp_gas_const_a * r_T);
     // carrier of air alone: ((1 - at) rho_a) / (1 - at) is rho_a
     if constexpr (sizeof(R) == 4) rho_c = rho_a;
-    else rho_c = ((R(1) - R(0) - at - R(0)) * rho_a + R(0)) / (R(1) - R(0) - at);
+    else rho_c = rdiv<R>((R(1) - R(0) - at - R(0)) * rho_a + R(0), R(1) - R(0) - at);
   } else {
     rho_c = P.rho_l;
   }
   R d = R(0);
   for (int i = 0; i < ns; ++i) d += al[i] * P.rho_s[i];
   R rho_m = (R(1) - at) * rho_c + d;
-  R inv_rhom = fdiv(R(1), rho_m);
-  R red_grav;
-  if constexpr (sizeof(R) == 4) red_grav = (rho_m - P.rho_a_amb) * inv_rhom * P.grav;
-  else red_grav = (rho_m - P.rho_a_amb) / rho_m * P.grav;
+  R inv_rhom, red_grav;
+  if constexpr (sizeof(R) == 4) {
+    inv_rhom = fdiv(R(1), rho_m);
+    red_grav = (rho_m - P.rho_a_amb) * inv_rhom * P.grav;
+  } else {
+    const Div64 vm = div64(rho_m);
+    inv_rhom = sp_heat_flag ? quot64(1.0, vm) : 0.0;
+    red_grav = quot64(rho_m - P.rho_a_amb, vm) * P.grav;
+  }
   R u2 = sq(r_u) + sq(r_v);
   m.Ri = (u2 > R(0)) ? rmin(cst<R>(1.0e15), fdiv(red_grav * r_h, u2)) : R(0);
   m.rho_m = rho_m;
@@ -321,7 +357,7 @@ __device__ __forceinline__ Mixt<R> mixt_var(const Phys<R>& P, const R* qpj, bool
     R cp_c;
     if (P.gas) {
       if constexpr (sizeof(R) == 4) cp_c = P.sp_heat_a;   // (x_c c_a) / x_c
-      else cp_c = (xc > P.thr_eps) ? ((xc - R(0)) * P.sp_heat_a + R(0)) / xc : P.sp_heat_a;
+      else cp_c = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_heat_a + R(0), xc) : P.sp_heat_a;
     } else {
       cp_c = P.sp_heat_l;
     }
@@ -363,7 +399,7 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
     R rho_a = fdiv(P.pres, P.sp_gas_const_a * r_T);
     // carrier of air alone: ((1 - at) rho_a) / (1 - at) is rho_a
     if constexpr (sizeof(R) == 4) rho_c = rho_a;
-    else rho_c = ((R(1) - R(0) - at - R(0)) * rho_a + R(0)) / (R(1) - R(0) - at);
+    else rho_c = rdiv<R>((R(1) - R(0) - at - R(0)) * rho_a + R(0), R(1) - R(0) - at);
   } else {
     rho_c = P.rho_l;
   }
@@ -371,12 +407,19 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
   R sa = R(0);
   for (int i = 0; i < ns; ++i) sa += arhos[i];
   R rho_m = alphac * rho_c + sa;
-  R inv_rhom = fdiv(R(1), rho_m);
+  R inv_rhom;
+  if constexpr (sizeof(R) == 4) {
+    inv_rhom = fdiv(R(1), rho_m);
+  } else {
+    const Div64 vm = div64(rho_m);
+    inv_rhom = quot64(1.0, vm);
+    m.red_grav = quot64(rho_m - P.rho_a_amb, vm) * P.grav;
+  }
   R xc = alphac * rho_c * inv_rhom;
   R cp_c;
   if (P.gas) {
     if constexpr (sizeof(R) == 4) cp_c = P.sp_heat_a;   // (x_c c_a) / x_c
-    else cp_c = (xc > P.thr_eps) ? ((xc - R(0)) * P.sp_heat_a + R(0)) / xc : P.sp_heat_a;
+    else cp_c = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_heat_a + R(0), xc) : P.sp_heat_a;
   } else {
     cp_c = P.sp_heat_l;
   }
@@ -395,7 +438,6 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
   m.rho_m = rho_m;
   m.rho_c = rho_c;
   if constexpr (sizeof(R) == 4) m.red_grav = (rho_m - P.rho_a_amb) * inv_rhom * P.grav;
-  else m.red_grav = (rho_m - P.rho_a_amb) / rho_m * P.grav;
   return m;
 }
 
@@ -409,7 +451,7 @@ __device__ __forceinline__ void local_speeds(const Phys<R>& P, const R* qpj, R r
   if (red_grav * r_h < R(0)) {
     vmin = vel; vmax = vel;
   } else {
-    R c = (dir == 1) ? sqrt(red_grav * r_h * gc) : sqrt(gc * red_grav * r_h);
+    R c = (dir == 1) ? rroot<R>(red_grav * r_h * gc) : rroot<R>(gc * red_grav * r_h);
     vmin = vel - c; vmax = vel + c;
   }
 }
@@ -437,9 +479,10 @@ __device__ __forceinline__ void eval_fluxes(const Phys<R>& P, const R* qcj, cons
     if (ns > 0 && flux[0] > R(0)) {
       R s = R(0);
       for (int i = 0; i < ns; ++i) s += flux[4 + i];
-      // flux[0] > 0 here: the FP32 form compares without the division
-      if (sizeof(R) == 4 ? s > flux[0] : s / flux[0] > R(1))
-        for (int i = 0; i < ns; ++i) flux[4 + i] = flux[4 + i] / s * flux[0];
+      // flux[0] > 0 here: s / flux[0], rounded, is above 1 exactly when s is
+      // above flux[0] (the next number above lies more than 2^-53 away)
+      if (s > flux[0])
+        for (int i = 0; i < ns; ++i) flux[4 + i] = rdiv<R>(flux[4 + i], s) * flux[0];
     }
   } else {
     for (int i = 0; i < nv; ++i) flux[i] = R(0);
@@ -480,7 +523,7 @@ __device__ __forceinline__ void expl_terms(const Phys<R>& P, const Geo<R>& g, co
   if (P.radial_source && arc_perim > R(0) && P.h_source > R(0)) {
     R t_coeff = t_coeff_src;
     if (t_coeff > R(0)) {
-      R h_dot = P.h_source * P.vel_source * arc_perim / P.cell_area;
+      R h_dot = rdiv<R>(P.h_source * P.vel_source * arc_perim, P.cell_area);
       e[0] = e[0] + t_coeff * h_dot * P.src_rho_m;
       e[1] = e[1] + t_coeff * h_dot * P.src_rho_m * P.vel_source * arc_nx;
       e[2] = e[2] + t_coeff * h_dot * P.src_rho_m * P.vel_source * arc_ny;
@@ -525,13 +568,14 @@ __device__ __forceinline__ void semi_impl_terms(const Phys<R>& P, const Geo<R>& 
   R r_h = qpj[0], r_u = qpj[nv], r_v = qpj[nv + 1];
   Mixt<R> m = mixt_var<R, NS>(P, qpj, false);
   R r_w = P.slope_corr ? (r_u * g.Bx + r_v * g.By) : R(0);
-  R mod_vel = sqrt(sq(r_u) + sq(r_v) + sq(r_w));
+  R mod_vel = rroot<R>(sq(r_u) + sq(r_v) + sq(r_w));
   if (P.rheo_model == 1 && mod_vel > R(0)) {
     R centr = P.curv ? (g.Bxx * sq(r_u) + cst<R>(2.0) * g.Bxy * r_u * r_v + g.Byy * sq(r_v)) : R(0);
-    R tt = P.mu * m.rho_m * (m.red_grav + centr) * r_h * sqrt(g.gc);
+    R tt = P.mu * m.rho_m * (m.red_grav + centr) * r_h * rroot<R>(g.gc);
     tt = rmax(R(0), tt);
-    si[1] = si[1] - tt * r_u / mod_vel;
-    si[2] = si[2] - tt * r_v / mod_vel;
+    const Divisor<R> vmod = divisor<R>(mod_vel);
+    si[1] = si[1] - quotient<R>(tt * r_u, vmod);
+    si[2] = si[2] - quotient<R>(tt * r_v, vmod);
   } else if (P.rheo_model == 11 && mod_vel > R(0)) {
     // grain diameter and density: Sauter mean and volume-weighted mean
     // (sauter_diameter, average_density_solids, constitutive_2d.f90:387-416)
@@ -539,7 +583,7 @@ __device__ __forceinline__ void semi_impl_terms(const Phys<R>& P, const Geo<R>& 
     R diam, rho_p;
     if (ns > 1) {
       R al[kMaxSolid], sa = R(0);
-      for (int i = 0; i < ns; ++i) { al[i] = P.alpha ? qpj[4 + i] : qpj[4 + i] / qpj[0]; sa += al[i]; }
+      for (int i = 0; i < ns; ++i) { al[i] = P.alpha ? qpj[4 + i] : rdiv<R>(qpj[4 + i], qpj[0]); sa += al[i]; }
       if (sa < P.thr_eps) {
         R sd = R(0), sr = R(0);
         for (int i = 0; i < ns; ++i) { sd += P.diam_s[i]; sr += P.rho_s[i]; }
@@ -547,9 +591,9 @@ __device__ __forceinline__ void semi_impl_terms(const Phys<R>& P, const Geo<R>& 
         rho_p = sr / R(ns);
       } else {
         R sdi = R(0), sar = R(0);
-        for (int i = 0; i < ns; ++i) { sdi += al[i] / P.diam_s[i]; sar += al[i] * P.rho_s[i]; }
-        diam = sa / sdi;
-        rho_p = sar / sa;
+        for (int i = 0; i < ns; ++i) { sdi += rdiv<R>(al[i], P.diam_s[i]); sar += al[i] * P.rho_s[i]; }
+        diam = rdiv<R>(sa, sdi);
+        rho_p = rdiv<R>(sar, sa);
       }
     } else {
       diam = P.diam_s[0];
@@ -559,14 +603,14 @@ __device__ __forceinline__ void semi_impl_terms(const Phys<R>& P, const Geo<R>& 
     R centr = P.curv ? (g.Bxx * sq(r_u) + cst<R>(2.0) * g.Bxy * r_u * r_v + g.Byy * sq(r_v)) : R(0);
     R vert = m.rho_m * (m.red_grav + centr) * hh;
     vert = rmax(vert, R(0));
-    R eff = rmax(R(0), vert * sqrt(g.gc));
+    R eff = rmax(R(0), vert * rroot<R>(g.gc));
     if (eff < P.thr_eps) eff = P.thr_eps;
-    const R shear = cst<R>(2.5) * mod_vel / (hh * sqrt(g.gc));
-    const R I = diam * shear / sqrt(eff / rho_p);
-    const R mu_I = (P.mu_s * P.I_0 + P.mu_2 * I + P.muI_inf * (I * I)) / (P.I_0 + I);
+    const R shear = rdiv<R>(cst<R>(2.5) * mod_vel, hh * rroot<R>(g.gc));
+    const R I = rdiv<R>(diam * shear, rroot<R>(rdiv<R>(eff, rho_p)));
+    const R mu_I = rdiv<R>(P.mu_s * P.I_0 + P.mu_2 * I + P.muI_inf * (I * I), P.I_0 + I);
     const R tt = mu_I * eff;
-    si[1] = si[1] - tt * (r_u / mod_vel);
-    si[2] = si[2] - tt * (r_v / mod_vel);
+    si[1] = si[1] - tt * rdiv<R>(r_u, mod_vel);
+    si[2] = si[2] - tt * rdiv<R>(r_v, mod_vel);
   }
 }
 
@@ -583,7 +627,7 @@ __device__ __forceinline__ bool rel_below(R d, R s, R tol) {
     const long long diff = d64_bits(d) - d64_bits(s * tol);
     if (diff > 8 || diff < -8) return diff < 0;
   }
-  return d / s < tol;
+  return rdiv<R>(d, s) < tol;
 }
 
 template <class R>
@@ -591,17 +635,17 @@ __device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos,
                                                R inv_kin_visc) {
   R inv_sqrt_C_D = R(1);
   if (rhos <= rhoc) return R(0);
-  R const_part = sqrt((cst<R>(4.0) / cst<R>(3.0)) * (rhos / rhoc - R(1)) * diam * P.grav);
+  R const_part = rroot<R>((cst<R>(4.0) / cst<R>(3.0)) * (rdiv<R>(rhos, rhoc) - R(1)) * diam * P.grav);
   R sv = const_part * inv_sqrt_C_D;
   R Rey = diam * sv * inv_kin_visc;
   if (Rey <= cst<R>(1000.0)) {
     for (int i = 1; i <= 20; ++i) {
       R sv_old = sv;
       if (P.collective)
-        inv_sqrt_C_D = sqrt(R(1) / (cst<R>(24.0) * (R(1) + cst<R>(0.15) * rpow<R>(Rey, cst<R>(0.687))) / Rey +
-                                    P.A_drag * (rlog<R>(Rey) - P.B_drag)));
+        inv_sqrt_C_D = rroot<R>(rdiv<R>(R(1), rdiv<R>(cst<R>(24.0) * (R(1) + cst<R>(0.15) * rpow<R>(Rey, cst<R>(0.687))), Rey) +
+                                                  P.A_drag * (rlog<R>(Rey) - P.B_drag)));
       else
-        inv_sqrt_C_D = sqrt(Rey / (cst<R>(24.0) * (R(1) + cst<R>(0.15) * rpow<R>(Rey, cst<R>(0.687)))));
+        inv_sqrt_C_D = rroot<R>(rdiv<R>(Rey, cst<R>(24.0) * (R(1) + cst<R>(0.15) * rpow<R>(Rey, cst<R>(0.687)))));
       sv = const_part * inv_sqrt_C_D;
       if (rel_below<R>(fabs(sv_old - sv), sv_old, cst<R>(1.0e-6))) return sv;
       Rey = diam * sv * inv_kin_visc;
@@ -630,32 +674,32 @@ __device__ __forceinline__ void mass_exchange(const Phys<R>& P, const R* qpj, R 
   R r_h = qpj[0], r_u = qpj[nv], r_v = qpj[nv + 1];
   R al[kMaxSolid];
   R at = R(0);
-  for (int i = 0; i < ns; ++i) { al[i] = P.alpha ? qpj[4 + i] : qpj[4 + i] / qpj[0]; at += al[i]; }
+  for (int i = 0; i < ns; ++i) { al[i] = P.alpha ? qpj[4 + i] : rdiv<R>(qpj[4 + i], qpj[0]); at += al[i]; }
   R r_w = P.slope_corr ? (r_u * Bx + r_v * By) : R(0);
   R mod_vel2 = sq(r_u) + sq(r_v) + sq(r_w);
   if (P.erosion_coeff > R(0)) {
     // Fagents & Baloga (2006) eq. 5 with the solid volume fraction
-    const R mod_vel = sqrt(mod_vel2);
+    const R mod_vel = rroot<R>(mod_vel2);
     const R tot = P.erosion_coeff * mod_vel * r_h * (R(1) - at);
     const R tot_solid = tot * (R(1) - P.erodible_porosity);
     for (int i = 0; i < ns; ++i) ers[i] = P.erodible_fract[i] * tot_solid;
   }
-  for (int i = 0; i < ns; ++i) ers[i] = rmax(R(0), rmin(ers[i], (erodible ? erodible[i] : R(0)) / dt));
+  for (int i = 0; i < ns; ++i) ers[i] = rmax(R(0), rmin(ers[i], rdiv<R>(erodible ? erodible[i] : R(0), dt)));
   R tot_solid_erosion = R(0);
   for (int i = 0; i < ns; ++i) tot_solid_erosion += ers[i];
-  R tot_erosion = tot_solid_erosion / (R(1) - P.erodible_porosity);
+  R tot_erosion = rdiv<R>(tot_solid_erosion, R(1) - P.erodible_porosity);
   R cont_erosion = tot_erosion * P.erodible_porosity;
   if (at <= P.alphastot_min) return;
   R r_T = qpj[3];
   Mixt<R> m = mixt_var<R, NS>(P, qpj, true);
-  R inv_kin_visc = R(1) / P.kin_visc_c;
+  R inv_kin_visc = rdiv<R>(R(1), P.kin_visc_c);
   R sdep = R(0);
   for (int i = 0; i < ns; ++i) {
     if (al[i] > R(0) && P.settling) {
       R sv = settling_velocity<R>(P, P.diam_s[i], P.rho_s[i], m.rho_c, inv_kin_visc);
       dep[i] = al[i] * sv * R(1);
-      dep[i] = dep[i] * rpow<R>(R(1) - rmin(R(1), at / alpha_max), hind_exp);
-      const R cap = r_h * al[i] / dt;
+      dep[i] = dep[i] * rpow<R>(R(1) - rmin(R(1), rdiv<R>(at, alpha_max)), hind_exp);
+      const R cap = rdiv<R>(r_h * al[i], dt);
       if (dep_limited && !(dep[i] < cap)) *dep_limited |= 1u << i;   // the whole class settles out
       dep[i] = rmin(dep[i], cap);
     }
@@ -665,12 +709,12 @@ __device__ __forceinline__ void mass_exchange(const Phys<R>& P, const R* qpj, R 
   for (int i = 0; i < ns; ++i) sal += al[i];
   R cpl = P.liquid ? P.loss_rate : R(0);
   cpl = cpl + P.coeff_porosity * sdep;
-  cpl = rmin(cpl, r_h * rmax(R(0), P.max_packing - sal) / dt);
-  cpl = rmin(cpl, (r_h * (R(1) - sal) - P.coeff_porosity * (r_h * sal - dt * sdep)) / dt);
+  cpl = rmin(cpl, rdiv<R>(r_h * rmax(R(0), P.max_packing - sal), dt));
+  cpl = rmin(cpl, rdiv<R>(r_h * (R(1) - sal) - P.coeff_porosity * (r_h * sal - dt * sdep), dt));
   R air_entr = R(0);
   if (P.entrain && r_h > R(0) && m.Ri > R(0)) {
-    R entr_coeff = cst<R>(0.075) / sqrt(R(1) + cst<R>(718.0) * rpow<R>(m.Ri, cst<R>(2.4)));
-    air_entr = entr_coeff * sqrt(mod_vel2);
+    R entr_coeff = rdiv<R>(cst<R>(0.075), rroot<R>(R(1) + cst<R>(718.0) * rpow<R>(m.Ri, cst<R>(2.4))));
+    air_entr = entr_coeff * rroot<R>(mod_vel2);
   }
   const R T_ers = P.erodible_deposit ? r_T : P.T_erodible;
   R rho_dep_tot = R(0), rho_ers_tot = R(0), s_dep = R(0), s_ers = R(0), dep_tot = R(0), ers_tot = R(0);
@@ -693,7 +737,7 @@ __device__ __forceinline__ void mass_exchange(const Phys<R>& P, const R* qpj, R 
              T_ers * (s_ers + P.rho_c_sub * m.cp_c * cont_erosion) +
              P.T_ambient * P.sp_heat_a * P.rho_a_amb * air_entr;
   for (int i = 0; i < ns; ++i) eqn[4 + i] = P.rho_s[i] * (ers[i] - dep[i]);
-  topo = (dep_tot - ers_tot) / (R(1) - P.erodible_porosity);
+  topo = rdiv<R>(dep_tot - ers_tot, R(1) - P.erodible_porosity);
 }
 
 // ---------------------------------------------------------------------------

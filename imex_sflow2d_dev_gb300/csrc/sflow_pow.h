@@ -1,21 +1,24 @@
 /*
- * sflow_pow.h -- x^y in FP64 with a quick first evaluation (device code).
+ * sflow_pow.h -- x^y of the FP64 form, with the bits of sfm_pow
+ * (sflow_math.h) and a fraction of its cost (device code).
  *
- * sfm_pow (sflow_math.h) carries some 600 FP64 operations of double-double
- * arithmetic; GB300 executes FP64 at 1/64 of the FP32 rate, and the settling
- * closure calls it once per fixed-point iteration, class and cell.  Here
- * x^y is first evaluated with tables to a relative error below 2^-68 (about
- * 70 FP64 operations); when the value is further than 2^-64 from every
- * rounding boundary of FP64, its rounding is that of the exact x^y, which
- * is also what sfm_pow returns (relative error below 2^-70 before its one
- * rounding); otherwise -- about once in a thousand arguments -- sfm_pow
- * itself is evaluated (A. Ziv, Fast evaluation of elementary mathematical
- * functions with correctly rounded last bit, ACM TOMS 17(3), 1991).  So both
- * functions give the same bits (tests/test_pow.py, tests/test_gpu_math.py).
- * Measured: 8 steps of a 512^2 FP64 current with settling of 2 classes 54.4 ->
- * 32.8 ms, 32 steps of a 360 x 180 eroding flood 107.9 -> 66.3 ms.
+ * sfm_pow carries some 600 FP64 operations of double-double arithmetic; GB300
+ * executes FP64 at 1/64 of the FP32 rate, and the settling closure calls it
+ * once per fixed-point iteration, class and cell.  sfm_pow_int, the function
+ * the kernels call, evaluates x^y in 64-bit fixed point on the integer
+ * pipes; sfm_pow_quick in about 70 FP64 operations to a relative error below
+ * 2^-68.  Each returns when its value is further than its error from every
+ * rounding boundary of FP64: the rounding is then that of the exact x^y,
+ * which is also what sfm_pow returns (relative error below 2^-70 before its
+ * one rounding).  The first passes the rest, about one argument in two
+ * hundred, to the second, and that about one in a thousand to sfm_pow (A. Ziv,
+ * Fast evaluation of elementary mathematical functions with correctly rounded
+ * last bit, ACM TOMS 17(3), 1991).  So all three give the same bits
+ * (tests/test_pow.py, tests/test_gpu_math.py).
+ * Measured: 8 steps of a 512^2 FP64 current with settling of 2 classes took
+ * 54.4 ms with sfm_pow, 32.8 ms with sfm_pow_quick.
  *
- * Method:
+ * Method of sfm_pow_quick:
  *  log x   x = 2^k m, m in [1, 2), c_i = 1/m rounded to 8 bits at the centre
  *          of the i-th of 128 intervals; r = m c - 1 is exact (|r| <= 2^-7,
  *          a multiple of 2^-60); log x = k ln 2 - log c + log1p(r).
@@ -366,6 +369,365 @@ SFM_FN double sfm_pow_quick(double x, double y) {
   const double u = SFM_ADD(s.hi, SFM_SUB(g, 0x1p-64)), v = SFM_ADD(s.hi, SFM_ADD(g, 0x1p-64));
   if (sfm_bits(u) != sfm_bits(v)) return sfm_pow_slow(x, y);
   return sfm_from_bits(sfm_bits(u) + ((int64_t)(n >> 7) << 52));
+}
+
+/* the FP64 evaluation, out of line */
+SFM_COLD double sfm_pow_quick_cold(double x, double y) { return sfm_pow_quick(x, y); }
+
+/*
+ * The same power on the integer pipes.  An FP64 instruction of a warp holds
+ * an SM's FP64 pipe for 16 cycles on GB300, in which the SM issues up to 64
+ * others, so 64-bit fixed point beats FP64 arithmetic: log2 x and 2^f by the
+ * reductions above with series in 64 x 64 -> 128 bit products (base 2, so
+ * that y log2 x splits into integer and fraction exactly), the result to
+ * 2^-61 (|y| < 1) or 2^-59 (|y| < 8).  The rounding test then leaves about
+ * one argument in two hundred (|y| < 1) to the FP64 evaluation above.
+ * log2 x = k + L_i + log2(1 + r), r = m c - 1 exact, L_i in [-1/2, 1/2] to
+ * 2^-64; log2(1 + r) = r P(r) to r^8 (next term below 2^-68); y log2 x exact
+ * in 128 bits; 2^f = 1 + f Q(f), |f| <= 2^-8, to f^6 (next below 2^-71).
+ * Coefficients: of P and Q at the scales 2^(62 - 6 n), so that a Horner step
+ * is one high product.
+ */
+#if defined(__CUDACC__)
+#define SFM_ITAB static __device__ const int64_t
+SFM_FN int64_t sfm_mulhi(int64_t a, int64_t b) { return __mul64hi(a, b); }
+SFM_FN int32_t sfm_mulhi32(int32_t a, int32_t b) { return __mulhi(a, b); }
+#else
+#define SFM_ITAB static const int64_t
+SFM_FN int64_t sfm_mulhi(int64_t a, int64_t b) { return (int64_t)(((__int128)a * b) >> 64); }
+SFM_FN int32_t sfm_mulhi32(int32_t a, int32_t b) { return (int32_t)(((int64_t)a * b) >> 32); }
+#endif
+/* per interval: L_i 2^63 (-log2 c, less 1 from the interval of 1/sqrt(2) on), 256 c */
+SFM_ITAB sfm_powi_log_tab[128 * 2] = {
+    52080352580344565LL, 255,
+    156856587611359393LL, 253,
+    262464388758716179LL, 251,
+    368917061291480011LL, 249,
+    476228232387282600LL, 247,
+    584411861601177296LL, 245,
+    638835303920586374LL, 244,
+    748354548482425863LL, 242,
+    858782676832593460LL, 240,
+    970134900679354152LL, 238,
+    1026162407023108733LL, 237,
+    1138930142077825653LL, 235,
+    1252661715613151172LL, 233,
+    1309894118242293459LL, 232,
+    1425102743535505569LL, 230,
+    1541317570432119309LL, 228,
+    1599807832071135499LL, 227,
+    1717565353665186919LL, 225,
+    1776837224931603046LL, 224,
+    1896178949527447616LL, 222,
+    1956253602797536653LL, 221,
+    2077222736812378418LL, 219,
+    2138122216557105918LL, 218,
+    2260763758429090961LL, 216,
+    2322511029776656571LL, 215,
+    2446871870455587345LL, 213,
+    2509490871181947108LL, 212,
+    2572405943934259308LL, 211,
+    2699135598006097888LL, 209,
+    2762955927049785547LL, 208,
+    2827083825132003070LL, 207,
+    2956274287476944212LL, 205,
+    3021342940842373362LL, 204,
+    3086731343173896505LL, 203,
+    3152442652505152648LL, 202,
+    3284846860330718215LL, 200,
+    3351546313759202669LL, 199,
+    3418581786003069540LL, 198,
+    3485956679806199380LL, 197,
+    3553674449863206093LL, 196,
+    3690152703675950302LL, 194,
+    3758920366278535087LL, 193,
+    3828045265094622256LL, 192,
+    3897531131076026346LL, 191,
+    3967381753930244064LL, 190,
+    4037600983360694007LL, 189,
+    4108192730339854449LL, 188,
+    4179160968416351941LL, 187,
+    4250509735057093000LL, 186,
+    4322243133025572372LL, 185,
+    4394365331797534366LL, 184,
+    4466880569015208631LL, 183,
+    4539793151981388594LL, 182,
+    -4610264577660106100LL, 181,
+    -4536544094927560092LL, 180,
+    -4462412911008301306LL, 179,
+    -4387866424172454937LL, 178,
+    -4312899954913613981LL, 177,
+    -4237508744186174972LL, 176,
+    -4161687951592454547LL, 175,
+    -4085432653517860093LL, 174,
+    -4008737841212318039LL, 173,
+    -3931598418816090440LL, 172,
+    -3854009201328034243LL, 171,
+    -3775964912514277691LL, 170,
+    -3697460182755204713LL, 169,
+    -3618489546828550505LL, 168,
+    -3618489546828550505LL, 168,
+    -3539047441626319689LL, 167,
+    -3459128203803142245LL, 166,
+    -3378726067353581513LL, 165,
+    -3297835161115802799LL, 164,
+    -3216449506198900170LL, 163,
+    -3216449506198900170LL, 163,
+    -3134563013331062591LL, 162,
+    -3052169480125638396LL, 161,
+    -2969262588262028797LL, 160,
+    -2885835900578206443LL, 159,
+    -2885835900578206443LL, 159,
+    -2801882858071513523LL, 158,
+    -2717396776804245214LL, 157,
+    -2632370844710368005LL, 156,
+    -2632370844710368005LL, 156,
+    -2546798118299558053LL, 155,
+    -2460671519254571926LL, 154,
+    -2373983830917780190LL, 153,
+    -2373983830917780190LL, 153,
+    -2286727694662502948LL, 152,
+    -2198895606144584904LL, 151,
+    -2198895606144584904LL, 151,
+    -2110479911429435337LL, 150,
+    -2021472802989534785LL, 149,
+    -2021472802989534785LL, 149,
+    -1931866315567174640LL, 148,
+    -1841652321896947459LL, 147,
+    -1841652321896947459LL, 147,
+    -1750822528282243838LL, 146,
+    -1659368470019735338LL, 145,
+    -1659368470019735338LL, 145,
+    -1567281506665531296LL, 144,
+    -1474552817136389425LL, 143,
+    -1474552817136389425LL, 143,
+    -1381173394639034911LL, 142,
+    -1381173394639034911LL, 142,
+    -1287134041420299103LL, 141,
+    -1192425363330425750LL, 140,
+    -1192425363330425750LL, 140,
+    -1097037764191508750LL, 139,
+    -1097037764191508750LL, 139,
+    -1000961439962619186LL, 138,
+    -904186372692749655LL, 137,
+    -904186372692749655LL, 137,
+    -806702324252248894LL, 136,
+    -806702324252248894LL, 136,
+    -708498829832937836LL, 135,
+    -708498829832937836LL, 135,
+    -609565191206587738LL, 134,
+    -509890469730899901LL, 133,
+    -509890469730899901LL, 133,
+    -409463479091552716LL, 132,
+    -409463479091552716LL, 132,
+    -308272777768273083LL, 131,
+    -308272777768273083LL, 131,
+    -206306661212243249LL, 130,
+    -206306661212243249LL, 130,
+    -103553153721468184LL, 129,
+    -103553153721468184LL, 129,
+    0LL, 128,
+};
+#define SFM_POWI_J 53
+/* 2^(j/128) 2^63 - 2^63 */
+SFM_ITAB sfm_powi_exp_tab[128] = {
+    0LL,
+    50081998086712172LL,
+    100435936470566771LL,
+    151063291760485868LL,
+    201965548583231959LL,
+    253144199626944055LL,
+    304600745684910150LL,
+    356336695699577385LL,
+    408353566806801173LL,
+    460652884380334596LL,
+    513236182076559376LL,
+    566105001879459730LL,
+    619260894145840423LL,
+    672705417650790365LL,
+    726440139633393050LL,
+    780466635842685220LL,
+    834786490583865063LL,
+    889401296764751326LL,
+    944312655942494694LL,
+    999522178370542806LL,
+    1055031483045860288LL,
+    1110842197756405188LL,
+    1166955959128863196LL,
+    1223374412676641067LL,
+    1280099212848120630LL,
+    1337132023075174828LL,
+    1394474515821947180LL,
+    1452128372633896118LL,
+    1510095284187105633LL,
+    1568376950337863663LL,
+    1626975080172509696LL,
+    1685891392057553038LL,
+    1745127613690063215LL,
+    1804685482148333994LL,
+    1864566743942822501LL,
+    1924773155067364938LL,
+    1985306481050670393LL,
+    2046168497008094253LL,
+    2107360987693692753LL,
+    2168885747552560160LL,
+    2230744580773450158LL,
+    2292939301341682950LL,
+    2355471733092339650LL,
+    2418343709763745508LL,
+    2481557075051243545LL,
+    2545113682661260179LL,
+    2609015396365664414LL,
+    2673264090056422201LL,
+    2737861647800547562LL,
+    2802809963895352094LL,
+    2868110942923994474LL,
+    2933766499811331593LL,
+    2999778559880072952LL,
+    3066149058907239977LL,
+    3132879943180931895LL,
+    3199973169557399849LL,
+    3267430705518430918LL,
+    3335254529229043726LL,
+    3403446629595497333LL,
+    3472009006323615108LL,
+    3540943669977425296LL,
+    3610252642038119995LL,
+    3679937954963334281LL,
+    3750001652246747201LL,
+    3820445788478006404LL,
+    3891272429402978156LL,
+    3962483651984324497LL,
+    4034081544462409340LL,
+    4106068206416535273LL,
+    4178445748826512875LL,
+    4251216294134564347LL,
+    4324381976307563277LL,
+    4397944940899612351LL,
+    4471907345114960866LL,
+    4546271357871263875LL,
+    4621039159863184816LL,
+    4696212943626343510LL,
+    4771794913601611379LL,
+    4847787286199755783LL,
+    4924192289866435379LL,
+    5001012165147548381LL,
+    5078249164754935673LL,
+    5155905553632440669LL,
+    5233983609022327877LL,
+    5312485620532062115LL,
+    5391413890201450318LL,
+    5470770732570147933LL,
+    5550558474745531858LL,
+    5630779456470941924LL,
+    5711436030194292929LL,
+    5792530561137059221LL,
+    5874065427363633862LL,
+    5956043019851064410LL,
+    6038465742559167353LL,
+    6121336012501023263LL,
+    6204656259813854727LL,
+    6288428927830289140LL,
+    6372656473150008452LL,
+    6457341365711787958LL,
+    6542486088865926258LL,
+    6628093139447068501LL,
+    6714165027847425056LL,
+    6800704278090387748LL,
+    6887713427904545824LL,
+    6975195028798103825LL,
+    7063151646133703529LL,
+    7151585859203652177LL,
+    7240500261305559181LL,
+    7329897459818383528LL,
+    7419780076278894114LL,
+    7510150746458545256LL,
+    7601012120440769623LL,
+    7692366862698690863LL,
+    7784217652173258204LL,
+    7876567182351805316LL,
+    7969418161347035739LL,
+    8062773311976437195LL,
+    8156635371842127113LL,
+    8251007093411131706LL,
+    8345891244096100955LL,
+    8441290606336461868LL,
+    8537207977680012398LL,
+    8633646170864958393LL,
+    8730608013902396020LL,
+    8828096350159242042LL,
+    8926114038441614409LL,
+    9024663953078665589LL,
+    9123748984006871116LL,
+};
+#define SFM_POWI_P0 (6653256548922161246LL)
+#define SFM_POWI_P1 (-51978566788454385LL)
+#define SFM_POWI_P2 (541443404046400LL)
+#define SFM_POWI_P3 (-6345039891169LL)
+#define SFM_POWI_P4 (79312998640LL)
+#define SFM_POWI_P5 (-1032721336)
+#define SFM_POWI_P6 (13831089)
+#define SFM_POWI_P7 (-189097)
+#define SFM_POWI_Q0 (3196577161300663915LL)
+#define SFM_POWI_Q1 (17310144115608349LL)
+#define SFM_POWI_Q2 (62492070775105LL)
+#define SFM_POWI_Q3 (169203916661LL)
+#define SFM_POWI_Q4 (366510056)
+#define SFM_POWI_Q5 (661577)
+
+/* x^y; the bits of sfm_pow(x, y) for every x and y */
+SFM_COLD double sfm_pow_int(double x, double y) {
+  const int64_t bx = sfm_bits(x), by = sfm_bits(y);
+  const int ey = (int)((by >> 52) & 0x7ff) - 1023;
+  /* x positive and normal, |y| in [2^-3, 8) */
+  if (bx < 0x0010000000000000LL || bx >= 0x7ff0000000000000LL || (unsigned)(ey + 3) > 5u) return sfm_pow_quick_cold(x, y);
+  const int i = (int)((bx >> 45) & 127);
+  const int k = (int)((bx >> 52) - 1023) + (i >= SFM_POWI_J ? 1 : 0);
+  const int64_t ya = ((by & 0x000fffffffffffffLL) | 0x0010000000000000LL) << (ey + 3);   /* |y| 2^55 */
+  /* |y log2 x| below 500 */
+  if (((int)(ya >> 55) + 1) * ((k < 0 ? -k : k) + 1) > 480) return sfm_pow_quick_cold(x, y);
+  const int64_t yf = by < 0 ? -ya : ya;
+  const int64_t c8 = SFM_LD(sfm_powi_log_tab + 2 * i + 1);
+  /* r 2^70 */
+  const int64_t rs = ((((bx & 0x000fffffffffffffLL) | 0x0010000000000000LL) * c8) - 0x1000000000000000LL) << 10;
+  const int32_t rh = (int32_t)(rs >> 32);
+  const int32_t p5 = SFM_POWI_P5 + sfm_mulhi32(rh, SFM_POWI_P6 + sfm_mulhi32(rh, SFM_POWI_P7));
+  int64_t p = SFM_POWI_P4 + sfm_mulhi32(rh, p5);
+  p = SFM_POWI_P3 + sfm_mulhi(rs, p);
+  p = SFM_POWI_P2 + sfm_mulhi(rs, p);
+  p = SFM_POWI_P1 + sfm_mulhi(rs, p);
+  p = SFM_POWI_P0 + sfm_mulhi(rs, p);
+  const int64_t L = SFM_LD(sfm_powi_log_tab + 2 * i) + ((sfm_mulhi(rs, p) + 16) >> 5);   /* (log2 x - k) 2^63 */
+  /* E = y log2 x at 2^118 in (eh, el) */
+  const uint64_t el0 = (uint64_t)yf * (uint64_t)L;
+  const int64_t eh0 = sfm_mulhi(yf, L);
+  const uint64_t kl = (uint64_t)yf * (uint64_t)(int64_t)k;
+  const int64_t kh = sfm_mulhi(yf, (int64_t)k);
+  const uint64_t el = el0 + (kl << 63);
+  int64_t eh = eh0 + (int64_t)((kl >> 1) | ((uint64_t)kh << 63)) + (el < el0 ? 1 : 0);
+  const int64_t n = (eh + 0x0000400000000000LL) >> 47;      /* 128 E rounded */
+  eh -= (int64_t)((uint64_t)n << 47);
+  const int64_t fs = (int64_t)(((uint64_t)eh << 16) | (el >> 48));   /* f 2^70 */
+  const int32_t fh = (int32_t)(fs >> 32);
+  int64_t q = SFM_POWI_Q3 + sfm_mulhi32(fh, SFM_POWI_Q4 + sfm_mulhi32(fh, SFM_POWI_Q5));
+  q = SFM_POWI_Q2 + sfm_mulhi(fs, q);
+  q = SFM_POWI_Q1 + sfm_mulhi(fs, q);
+  q = SFM_POWI_Q0 + sfm_mulhi(fs, q);
+  const int64_t fq = sfm_mulhi(fs, q);                      /* (2^f - 1) 2^68 */
+  const uint64_t T = (uint64_t)SFM_LD(sfm_powi_exp_tab + (int)(n & 127)) + 0x8000000000000000ULL;
+  uint64_t G = T + (uint64_t)((sfm_mulhi((int64_t)(T >> 1), fq) + 4) >> 3);   /* 2^(f + j/128) 2^63 */
+  int e = (int)(n >> 7) + 1022;
+  if (!(G >> 63)) {
+    G <<= 1;
+    e -= 1;
+  }
+  /* G is off by at most 1.1 |y| ln 2 2^(j/128) units of 2^-63 from log2 x and
+     1.2 from the table and the last product (twice that in units below 1):
+     3.3 for |y| < 1, 13 for |y| < 8.  Round unless the midpoint is that close */
+  const int err = ey < 0 ? 4 : 14;
+  const int low = (int)(G & 2047u) - 1024;
+  if (low <= err && low >= -err) return sfm_pow_quick_cold(x, y);
+  return sfm_from_bits((int64_t)(((uint64_t)e << 52) + (G >> 11) + (low > 0 ? 1u : 0u)));
 }
 
 #endif /* SFLOW_POW_H */

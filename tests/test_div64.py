@@ -1,9 +1,11 @@
-"""Quotients by a shared divisor and integer comparisons of the FP64 kernels
+"""Integer division, square root and comparisons of the FP64 kernels
 (imex_sflow2d_dev_gb300/csrc/sflow_div64.cuh), compiled for the host: the
-bits of the plain division and the answers of the plain comparisons, on
+bits of the FP64 operations and the answers of the FP64 comparisons, on
 random bit patterns, mantissas next to rounding boundaries (a quotient times
 the divisor, +-2 ulp; divisors of nearly all ones), zeros of both signs,
-infinities, NaN, subnormals and the ends of the range."""
+infinities, NaN, subnormals and the ends of the range; squares +-2 ulp for
+the root.  The float estimates that start the iterations are shifted by up
+to 2^-22, more than the device's approximations are off."""
 import os
 import shutil
 import subprocess
@@ -15,6 +17,8 @@ CSRC = os.path.join(os.path.dirname(__file__), "..", "imex_sflow2d_dev_gb300", "
 PROG = r'''
 #include <cstdio>
 #include <cmath>
+static int noise = 0;
+#define D64_SEED_NOISE noise
 #include "sflow_div64.cuh"
 using namespace sflow;
 static uint64_t s = 88172645463325252ULL;
@@ -28,6 +32,9 @@ static long check(double a, double d) {
   bad += (a < 0) != d64_neg(a);
   bad += (a == 0) != d64_zero(a);
   bad += (a > 1.5) != d64_gt_pos(a, 1.5);
+  bad += d64_bits(ddiv64(a, d)) != d64_bits(x) && !(x != x);
+  const double r = dsqrt64(a), r0 = sqrt(a);
+  bad += d64_bits(r) != d64_bits(r0) && !(r != r && r0 != r0);
   const double u = fabs(a), v = fabs(d), m = u > v ? u : v, n = d64_from(d64_absmax(d64_bits(u), d64_bits(v)));
   bad += d64_bits(m) != d64_bits(n) && !(m != m && n != n);
   return bad;
@@ -39,12 +46,14 @@ int main() {
   for (double a : sp) for (double d : sp) bad += check(a, d);
   for (long i = 0; i < 2000000; ++i) {
     double a, d;
-    switch (i % 6) {
+    noise = (int)(rn() % 1024) - 512;
+    switch (i % 7) {
       case 0: a = d64_from((long long)rn()); d = d64_from((long long)rn()); break;
       case 1: a = unit(); d = unit(); break;
       case 2: d = unit(); a = unit() * d; a = d64_from(d64_bits(a) + (long long)(rn() % 5) - 2); break;
       case 3: d = 2.0 - (double)(rn() % 64 + 1) * 0x1p-52; a = unit(); break;
       case 4: d = (double)(rn() % 1000 + 1); a = (double)(rn() % 100000) - 50000.0; break;
+      case 5: d = unit(); a = unit(); a = a * a; if (i & 1) a *= 2.0; a = d64_from(d64_bits(a) + (long long)(rn() % 5) - 2); break;
       default: a = sp[rn() % 20]; d = unit(); break;
     }
     bad += check(a, d);

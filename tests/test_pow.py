@@ -1,8 +1,8 @@
 """x^y of the FP64 kernels (imex_sflow2d_dev_gb300/csrc/sflow_pow.h): its
-tables recomputed from exact arithmetic, and its bits against those of
-sfm_pow (sflow_math.h) on the host, over the closures' argument ranges, near
-1, at random bit patterns and at the C99 special values.  Both functions
-round the exact power, so no bit may differ."""
+tables recomputed from exact arithmetic, and the bits of its FP64 and integer
+evaluations against those of sfm_pow (sflow_math.h) on the host, over the closures' argument ranges, near
+1, at random bit patterns and at the C99 special values.  All of
+them round the exact power, so no bit may differ."""
 import os
 import re
 import shutil
@@ -41,14 +41,43 @@ def test_tables_are_the_exact_values_split():
     assert d["SFM_POW_INV_L"] == float(128 / ln2)
 
 
+def test_integer_tables_and_coefficients_are_the_rounded_exact_values():
+    getcontext().prec = 60
+    text = open(os.path.join(CSRC, "sflow_pow.h")).read()
+    ln2 = Decimal(2).ln()
+
+    def ints(name):
+        body = re.search(name + r"\[[^\]]*\] = \{(.*?)\};", text, re.S).group(1)
+        return [int(v.strip().rstrip("L")) for v in body.replace("\n", " ").split(",") if v.strip()]
+
+    def rnd(v):
+        return int(v.to_integral_value())
+    t, first = ints("sfm_powi_log_tab"), None
+    for i in range(128):
+        c8 = rnd(256 / (1 + (Decimal(i) + Decimal("0.5")) / 128))
+        v = -(Decimal(c8) / 256).ln() / ln2
+        if v > Decimal("0.5"):
+            first, v = (i if first is None else first), v - 1
+        assert t[2 * i:2 * i + 2] == [rnd(v * 2 ** 63), c8]
+    assert ints("sfm_powi_exp_tab") == [rnd(((ln2 * j / 128).exp() - 1) * 2 ** 63) for j in range(128)]
+    d = {k: int(v) for k, v in re.findall(r"#define SFM_POWI_([JPQ]\d?) \(?(-?\d+)", text)}
+    assert d["J"] == first
+    f = 1
+    for n in range(8):
+        assert d[f"P{n}"] == rnd((-1) ** n / ln2 / (n + 1) * Decimal(2) ** (62 - 6 * n))
+        f *= n + 1
+        if n < 6:
+            assert d[f"Q{n}"] == rnd(ln2 ** (n + 1) / f * Decimal(2) ** (62 - 6 * n))
+
+
 PROG = r'''
 #include <stdio.h>
 #include "sflow_pow.h"
 static uint64_t s = 88172645463325252ULL;
 static uint64_t rn(void) { s ^= s << 13; s ^= s >> 7; s ^= s << 17; return s; }
 static long differ(double x, double y) {
-  const double a = sfm_pow(x, y), b = sfm_pow_quick(x, y);
-  return sfm_bits(a) != sfm_bits(b) && !(a != a && b != b);
+  const double a = sfm_pow(x, y), b = sfm_pow_quick(x, y), c = sfm_pow_int(x, y);
+  return (sfm_bits(a) != sfm_bits(b) || sfm_bits(a) != sfm_bits(c)) && !(a != a && b != b && c != c);
 }
 int main(void) {
   const double ys[] = {0.687, 4.65, 2.4, 0.5, -1.3, 3.0, 1.0, 17.25, -40.0, 0.0};
