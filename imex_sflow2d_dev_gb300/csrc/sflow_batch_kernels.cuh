@@ -100,8 +100,10 @@ struct BatchArgs {
 constexpr int kBatchCandThreads = 256;
 // 128-thread stage blocks (4 per SM at least): the bound then leaves the
 // per-cell Newton its registers without spills; measured 5 % faster than
-// 256-thread blocks held to 64 registers
-constexpr int kBatchStageThreads = 128;
+// 256-thread blocks held to 64 registers.  FP64: 64 threads, 4 blocks per SM
+// (see StageShape).
+template <class R>
+constexpr int kBatchStageThreads = sizeof(R) == 4 ? 128 : 64;
 
 __device__ __forceinline__ int entry_slot(unsigned long long e) { return (int)(e >> 48); }
 __device__ __forceinline__ unsigned entry_gen(unsigned long long e) { return (unsigned)(e >> 32) & 0xffffu; }
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(kBatchCandThreads) k_b_dt(BatchArgs<R> b) {
 // holding the tile's byte; the Newton counters are summed per run over the
 // lanes of a warp that share it.
 template <class R, int NS, int TH>
-__global__ void __launch_bounds__(kBatchStageThreads, sizeof(R) == 4 ? 4 : 1) k_b_stage2(BatchArgs<R> b) {
+__global__ void __launch_bounds__(kBatchStageThreads<R>, 4) k_b_stage2(BatchArgs<R> b) {
   step_kernel_entry();
   BatchCtl* ctl = b.ctl;
   const unsigned n = min(ctl->ncells, b.cells_cap);

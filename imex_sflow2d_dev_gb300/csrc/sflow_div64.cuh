@@ -14,6 +14,9 @@
 // kernels' bits).  About 60 instructions a quotient, 25 for a further one by
 // the same divisor.  Operands outside the middle of the range, infinities
 // and NaN take the FP64 operation itself.
+// Measured with the power on the integer pipes (sflow_pow.h), before -> after:
+// 512^2 current with settling, 8 steps, 23.9 -> 14.1 ms; 200^2 dam break to
+// 10 s 115.0 -> 48.6 ms; 360 x 180 eroding flood, 32 steps, 42.9 -> 24.3 ms.
 // Newton's iteration for reciprocals in fixed point with a remainder
 // correction: M. J. Flynn, On division by functional iteration, IEEE Trans.
 // Comput. C-19(8), 1970.

@@ -41,13 +41,27 @@ struct TileShape {
   static constexpr int FLUX_THREADS = (TX * (TH + 1) + 31) / 32 * 32;
   // resident blocks per SM the persistent flux kernel is compiled for
   static constexpr int FLUX_MIN_BLOCKS = (TH >= 16) ? 2 : (TH >= 8 ? 4 : 6);
-  // pointwise kernels: 32 x 8 threads, one cell each (a single run's
-  // blocks cover 32 x 8 cells; a batched block walks a tile 8 rows at a time)
-  static constexpr int STAGE_THREADS = TX * 8;
-  static constexpr int STAGE_MIN_BLOCKS = 5;
   static constexpr int MASK_THREADS = TX * TH;
 };
 constexpr int kTileHDefault = 8;
+
+// Thread blocks of a single run's pointwise kernels: 32 x ROWS cells, one
+// cell each, of one tile (or half a tile of 32 x 4).
+//  FP32: 8 rows, 6 blocks per SM (40 registers): the stage waits on memory,
+//        and more warps hide more of it.
+//  FP64: 2 rows, 4 blocks per SM (255 registers).  The stage is bound by
+//        FP64 instructions and the latency of their chains, both varying
+//        tenfold between warps (Newton and settling iterations, wet or dry),
+//        so small blocks spread over the SMs best; held to 168 registers for
+//        12 warps per SM its spills cost more than the warps gave (512^2
+//        current 1.04 against 1.14 ms, eroding flood 0.36 against 0.39; 8
+//        rows, 1 block: 1.05 and 0.42).
+template <class R>
+struct StageShape {
+  static constexpr int ROWS = sizeof(R) == 4 ? 8 : 2;
+  static constexpr int THREADS = TX * ROWS;
+  static constexpr int MIN_BLOCKS = sizeof(R) == 4 ? 6 : 4;
+};
 
 // flag byte bits
 constexpr uint8_t F_SC_MASK = 0x3;  // source_cell (0, 1 ring interior, 2 ring boundary)
@@ -1743,22 +1757,20 @@ __device__ __forceinline__ int stage2_cell(const KArgs<R>& a, int mode, int j, i
 // neighbours across those edges can gain active cells.  0xff: unknown.
 constexpr uint8_t TW_ANY = 1, TW_W = 2, TW_E = 4, TW_S = 8, TW_N = 16;
 
-// single run: one block per 32 x 8 cells (grid tiles_x x ceil(ny/8)); the
-// activity byte is the one of the 32 x TH tile holding the block.  The FP32
-// form is compiled for 6 resident blocks per SM (40 registers): the kernel
-// waits on memory, and more warps hide more of it.
+// single run: one block per 32 x ROWS cells (grid tiles_x x ceil(ny/ROWS));
+// the activity byte is the one of the 32 x TH tile holding the block.
 template <class R, int NS, int TH>
-__global__ void __launch_bounds__(TileShape<TH>::STAGE_THREADS, sizeof(R) == 4 ? 6 : 1)
-    k_stage2(KArgs<R> a, int mode) {
+__global__ void __launch_bounds__(StageShape<R>::THREADS, StageShape<R>::MIN_BLOCKS) k_stage2(KArgs<R> a, int mode) {
+  constexpr int ROWS = StageShape<R>::ROWS;
   step_kernel_entry();
   if (!a.st->run_step) return;
-  const int kk = blockIdx.y * 8 + threadIdx.x / TX;
+  const int kk = blockIdx.y * ROWS + threadIdx.x / TX;
   // inactive, or left unchanged (k_flux's dry tiles, k_mask's dry border)
   auto skipped = [](uint8_t ta) { return ta == 0 || ta == 2 || ta == TILE_DRY_BORDER; };
   int tile;
   bool run = true;
   if constexpr (TH >= 8) {
-    tile = (blockIdx.y * 8 / TH) * gridDim.x + blockIdx.x;
+    tile = (blockIdx.y * ROWS / TH) * gridDim.x + blockIdx.x;
     if (skipped(a.tile_active[tile])) return;
   } else {
     // 32 x 4 tiles: the block's two halves belong to two tiles
@@ -1790,17 +1802,18 @@ __global__ void __launch_bounds__(TileShape<TH>::STAGE_THREADS, sizeof(R) == 4 ?
 // per stage); qs holds the state of the running stage.
 // ---------------------------------------------------------------------------
 template <class R, int NS, int TH>
-__global__ void __launch_bounds__(TileShape<TH>::STAGE_THREADS) k_stage(KArgs<R> a, int irk) {
+__global__ void __launch_bounds__(StageShape<R>::THREADS, sizeof(R) == 4 ? 1 : 4) k_stage(KArgs<R> a, int irk) {
+  constexpr int ROWS = StageShape<R>::ROWS;
   step_kernel_entry();
   constexpr int nv = 4 + NS;
   RunState* st = a.st;
   if (!st->run_step) return;
   if constexpr (TH >= 8) {
-    if (!a.tile_active[(blockIdx.y * 8 / TH) * gridDim.x + blockIdx.x]) return;
+    if (!a.tile_active[(blockIdx.y * ROWS / TH) * gridDim.x + blockIdx.x]) return;
   }
   const Grid<R>& g = a.g;
   const int j = blockIdx.x * TX + threadIdx.x % TX;
-  const int k = blockIdx.y * 8 + threadIdx.x / TX;
+  const int k = blockIdx.y * ROWS + threadIdx.x / TX;
   unsigned status = 0;
   int nit = 0;
   if (j < g.nx && k < g.ny && (TH >= 8 || a.tile_active[(k / TH) * gridDim.x + blockIdx.x])) {
@@ -1838,17 +1851,18 @@ __global__ void __launch_bounds__(TileShape<TH>::STAGE_THREADS) k_stage(KArgs<R>
 
 // assemble_sol (solver_2d.f90:1342-1630) + erosion/deposition + maxima
 template <class R, int NS, int TH>
-__global__ void __launch_bounds__(TileShape<TH>::STAGE_THREADS) k_assemble(KArgs<R> a) {
+__global__ void __launch_bounds__(StageShape<R>::THREADS, sizeof(R) == 4 ? 1 : 4) k_assemble(KArgs<R> a) {
+  constexpr int ROWS = StageShape<R>::ROWS;
   step_kernel_entry();
   constexpr int nv = 4 + NS;
   RunState* st = a.st;
   if (!st->run_step) return;
   if constexpr (TH >= 8) {
-    if (!a.tile_active[(blockIdx.y * 8 / TH) * gridDim.x + blockIdx.x]) return;
+    if (!a.tile_active[(blockIdx.y * ROWS / TH) * gridDim.x + blockIdx.x]) return;
   }
   const Grid<R>& g = a.g;
   const int j = blockIdx.x * TX + threadIdx.x % TX;
-  const int k = blockIdx.y * 8 + threadIdx.x / TX;
+  const int k = blockIdx.y * ROWS + threadIdx.x / TX;
   unsigned status = 0;
   if (j < g.nx && k < g.ny && (TH >= 8 || a.tile_active[(k / TH) * gridDim.x + blockIdx.x])) {
     const int64_t c = cidx(g, j, k);

@@ -13,11 +13,12 @@
 //  * only the columns hu and hv are perturbed, so q(1), q(4) and the solid
 //    masses, and every quantity formed from them alone, stay real;
 //  * divisions and square roots run on the integer pipes, and the quotients
-//    by one divisor share its reciprocal (sflow_div64.cuh); the real divisors of the two columns equal those of the real
-//    evaluation unless a perturbation reaches them (tested on the bits);
+//    by one divisor share its reciprocal (sflow_div64.cuh); the real
+//    divisors of the two columns equal those of the real evaluation unless a
+//    perturbation reaches them (tested on the bits);
 //  * the end-of-iteration residual is that of the next iteration's start;
-//  * the line search's slope, step bound and least step are formed only
-//    when the full step is refused, the largest step only past 99 n_vars;
+//  * the line search's least step is formed only when a step is refused, its
+//    largest step only past 99 n_vars;
 //  * comparisons and maxima are integer ones.
 // Measured: 8 steps of the 512^2 current with settling (96,000 wet cells, 2.9
 // iterations each) 32.8 -> 23.9 ms, 32 steps of a 360 x 180 eroding flood
@@ -181,49 +182,40 @@ __device__ __forceinline__ void friction_real(const Phys<double>& P, double Bx, 
   }
 }
 
-// imaginary parts of the friction terms at the state of f with q(1 + COL)
-// perturbed by i e
-template <int COL>
+// imaginary parts of the friction terms at the state of f with hu (col = 0)
+// or hv (col = 1) perturbed by i e; one copy of the code for both columns
 __device__ __forceinline__ void friction_imag(const Phys<double>& P, double Bx, double By, const Div64& dxi,
-                                              const FrictPoint& f, double q1, double q2, double q3, double e,
+                                              const FrictPoint& f, int col, double q1, double q2, double q3, double e,
                                               double& im1, double& im2) {
   im1 = 0.0;
   im2 = 0.0;
   if (!f.live) return;
-  const Cplx a = (COL == 0) ? Cplx{q1, e} : Cplx{q1, 0.0};
-  const Cplx b = (COL == 1) ? Cplx{q2, e} : Cplx{q2, 0.0};
+  const double e1 = col ? 0.0 : e, e2 = col ? e : 0.0;
   // mixture density and reduced gravity: complex through the temperature
   Cplx rho{f.rho, 0.0}, rg{f.rg, 0.0};
   if (P.gas && P.energy && !f.film) {
-    const double pr = (COL == 0) ? q1 : q2;
+    const double pr = col ? q2 : q1, ot = col ? q1 : q2;
     const double two = pr * e + e * pr;
-    const double s = (COL == 0) ? (q1 * q1 - e * e) + q2 * q2 : q1 * q1 + (q2 * q2 - e * e);
+    // the perturbed square first or second in the sum: the same sum
+    const double s = (pr * pr - e * e) + ot * ot;
     const double nre = q3 - 0.5 * s * f.inv;
     const double nim = 0.0 - 0.5 * two * f.inv;
     const double Tre = quot64(nre, f.dT);
-    if (!(Tre <= 0.0)) {
-      const double Tim = quot64(nim, f.dT);
-      const Cplx ir{f.dinv + f.xc * (f.Rc * Tre * P.inv_pres), f.xc * (f.Rc * Tim * P.inv_pres)};
-      rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.rho);
-    } else {
-      const Cplx ir{f.dinv + f.xc * (f.Rc * P.T_ambient * P.inv_pres), 0.0};
-      rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.rho);
-    }
+    const bool low = Tre <= 0.0;
+    const double Tim = low ? 0.0 : quot64(nim, f.dT);
+    const Cplx ir{f.dinv + f.xc * (f.Rc * (low ? P.T_ambient : Tre) * P.inv_pres), f.xc * (f.Rc * Tim * P.inv_pres)};
+    rho = cdiv(Cplx{1.0, 0.0}, ir, f.dinvr, 1.0, f.rho);
     const Cplx qr = cdiv(Cplx{rho.re - P.rho_a_amb, rho.im}, rho, f.drho, f.nrg, f.qrg);
     rg = Cplx{qr.re * P.grav, qr.im * P.grav};
   }
-  Cplx u, v;
-  if (f.film) {
-    u = Cplx{quot64(f.s0 * a.re, f.den), quot64(f.s0 * a.im, f.den)};
-    v = Cplx{quot64(f.s0 * b.re, f.den), quot64(f.s0 * b.im, f.den)};
-  } else {
-    u = Cplx{f.u, a.im * f.inv};
-    v = Cplx{f.v, b.im * f.inv};
-  }
+  // the velocities: the imaginary part of the perturbed one; a film's real
+  // parts are those of the real evaluation (the same products and quotients)
+  const Cplx u{f.u, f.film ? quot64(f.s0 * e1, f.den) : e1 * f.inv};
+  const Cplx v{f.v, f.film ? quot64(f.s0 * e2, f.den) : e2 * f.inv};
   Cplx w{0.0, 0.0};
   if (P.slope_corr) w = Cplx{f.w, u.im * Bx + v.im * By};
-  const Cplx hz = (COL == 0) ? Cplx{(u.re * u.re - u.im * u.im) + v.re * v.re, u.re * u.im + u.im * u.re}
-                             : Cplx{u.re * u.re + (v.re * v.re - v.im * v.im), v.re * v.im + v.im * v.re};
+  const Cplx hz{(u.re * u.re - u.im * u.im) + (v.re * v.re - v.im * v.im),
+                (u.re * u.im + u.im * u.re) + (v.re * v.im + v.im * v.re)};
   const Cplx m2{hz.re + (w.re * w.re - w.im * w.im), hz.im + (w.re * w.im + w.im * w.re)};
   const Cplx mod = csqrt64(m2, f.m2, f.mod, f.dmod);
   if (d64_zero(mod.re)) return;
@@ -269,74 +261,117 @@ __device__ __forceinline__ long long newton_maxf(const double* f) {
 
 // solve_rk_step (normalize_q = T, normalize_f = F, opt_search_NL = T;
 // implicit set {hu, hv}); returns the iterations used (kMaxNewton + 1 when
-// the limit was reached)
+// the limit was reached).  The line search's cubic model never chooses its
+// step: its minimiser is capped at half the last step and the step kept above
+// the same half (solver_2d.f90:2205-2222), so after the first refusal, which
+// follows the quadratic model, the step is halved.  One loop evaluates the closure for every purpose, so that the
+// code holds it once (the kernel's code exceeds the instruction cache).
 template <int NS>
 __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
   constexpr int nv = 4 + NS;
-  const double STPMX = 100.0, TOLF = 1.0e-10, TOLMIN = 1.0e-6, TOLX = kEps;
+  const double STPMX = 100.0, TOLF = 1.0e-10, TOLX = kEps;
   const Phys<double>& P = *c.P;
   double org[nv], rel[nv], f[nv], p[nv], xo[nv], dtR[nv];
-  double scal_f, nh1, nh2;
+  double scal_f = 0.0, scal_old = 0.0, slope = 0.0, alam = 1.0, alamin = -1.0, nh1, nh2;
   FrictPoint fp;
   Div64 dxi{};
   if (P.rheo_model == 1) dxi = div64(P.xi);
   const double h = nv * kEps, one_by_h = 1.0 / h, dta = c.dt * c.a_diag;
-  bool check = false;
 #pragma unroll
   for (int i = 0; i < nv; ++i) dtR[i] = c.dt * c.Rj[i];
-  friction_real<NS>(P, c.Bx, c.By, dxi, qj, fp, nh1, nh2);
-  newton_residual<NS>(c, dtR, qj, nh1, nh2, f, scal_f);
-  if (newton_maxf<NS>(f) < d64_bits(TOLF)) return 1;
-  if (!isfinite(scal_f)) return kMaxNewton + 1;   // NaN/Inf state: give up at once
-  // the Jacobian's state is rel * org, which may differ from qj in the last bit
-  bool same = true;
+  enum { START, SCALED, FIRST, TRIAL } phase = START;
+  int it = 0;
+#pragma unroll 1
+  for (;;) {
+    friction_real<NS>(P, c.Bx, c.By, dxi, qj, fp, nh1, nh2);
+    if (phase != SCALED) newton_residual<NS>(c, dtR, qj, nh1, nh2, f, scal_f);
+    if (phase == START) {
+      if (newton_maxf<NS>(f) < d64_bits(TOLF)) return 1;
+      if (!isfinite(scal_f)) return kMaxNewton + 1;   // NaN/Inf state: give up at once
+      // the Jacobian's state is rel * org, which may differ from qj in the last bit
+      bool same = true;
 #pragma unroll
-  for (int i = 0; i < nv; ++i) {
-    org[i] = d64_lt(1.0e-3, fabs(qj[i])) ? fabs(qj[i]) : 1.0e-3;
-    rel[i] = ddiv64(qj[i], org[i]);
-    xo[i] = rel[i] * org[i];
-    same = same && d64_bits(xo[i]) == d64_bits(qj[i]);
-  }
-  if (!same) {
-    double n1, n2;
-    friction_real<NS>(P, c.Bx, c.By, dxi, xo, fp, n1, n2);
+      for (int i = 0; i < nv; ++i) {
+        org[i] = d64_lt(1.0e-3, fabs(qj[i])) ? fabs(qj[i]) : 1.0e-3;
+        rel[i] = ddiv64(qj[i], org[i]);
+        const double x = rel[i] * org[i];
+        same = same && d64_bits(x) == d64_bits(qj[i]);
+        qj[i] = x;
+      }
+      if (!same) {
+        phase = SCALED;
+        continue;
+      }
+    } else if (phase != SCALED) {
+      if (phase == TRIAL && (d64_lt(0.9 * scal_old, scal_f) || (d64_bits(scal_f) & kD64Abs) > kD64Inf)) {
+        // refused: a shorter step, or stop at the old point (where the step
+        // test below holds) when it is below the least step TOLX / max |p|
+        if (alamin < 0.0) {
+          double mx = 0.0;
 #pragma unroll
-    for (int i = 0; i < nv; ++i) qj[i] = xo[i];
-  }
-  for (int it = 1; it <= kMaxNewton; ++it) {
-    // here qj = rel * org, fp is the closure at qj, f the residual (of the
-    // unscaled start state in the first iteration)
-    double j11, j21, j12, j22;
-    friction_imag<0>(P, c.Bx, c.By, dxi, fp, qj[1], qj[2], qj[3], h * org[1], j11, j21);
-    friction_imag<1>(P, c.Bx, c.By, dxi, fp, qj[1], qj[2], qj[3], h * org[2], j12, j22);
-    const double s11 = org[1] - dta * (j11 * one_by_h), s12 = 0.0 - dta * (j12 * one_by_h);
-    const double s21 = 0.0 - dta * (j21 * one_by_h), s22 = org[2] - dta * (j22 * one_by_h);
+          for (int i = 0; i < nv; ++i) {
+            const double ax = fabs(xo[i]), t = ddiv64(fabs(p[i]), ax > 1.0 ? ax : 1.0);
+            if (i == 0 || t > mx) mx = t;
+          }
+          alamin = ddiv64(TOLX, mx);
+        }
+        const bool stop = alam < alamin;
+        const double quad = (alam == 1.0) ? -slope / (2.0 * (scal_f - scal_old - slope)) : 0.0;
+        alam = (quad > 0.5 * alam) ? quad : 0.5 * alam;
+#pragma unroll
+        for (int i = 0; i < nv; ++i) {
+          rel[i] = stop ? xo[i] : xo[i] + alam * p[i];
+          qj[i] = rel[i] * org[i];
+        }
+        if (stop) return it;
+        continue;
+      }
+      if (newton_maxf<NS>(f) < d64_bits(TOLF)) return it;
+      // |step| < TOLX max(|rel|, 1) in every component: TOLX is a power of
+      // two, so the product is exact and orders as the quotient does (a NaN
+      // component is forgotten when a later one is a number, as the maximum
+      // forgets it)
+      bool small = true, was_nan = false;
+#pragma unroll
+      for (int i = 0; i < nv; ++i) {
+        const double ar = fabs(rel[i]), st = fabs(rel[i] - xo[i]);
+        small = (small || was_nan) && d64_lt(st, TOLX * (d64_lt(1.0, ar) ? ar : 1.0));
+        was_nan = d64_bits(st) > kD64Inf || (d64_bits(st) == kD64Inf && d64_bits(ar) == kD64Inf);
+      }
+      if (small) return it;
+      // the next iteration's first test
+      if (!isfinite(scal_f)) return kMaxNewton + 1;
+    }
+    // the next direction; qj = rel * org, fp is the closure at qj, f the
+    // residual (of the unscaled start state in the first iteration)
+    if (++it > kMaxNewton) return kMaxNewton + 1;
+    double j1[2], j2[2];
+#pragma unroll 1
+    for (int col = 0; col < 2; ++col) {
+      double a1, a2;
+      friction_imag(P, c.Bx, c.By, dxi, fp, col, qj[1], qj[2], qj[3], h * (col ? org[2] : org[1]), a1, a2);
+      if (col) { j1[1] = a1; j2[1] = a2; }
+      else { j1[0] = a1; j2[0] = a2; }
+    }
+    const double s11 = org[1] - dta * (j1[0] * one_by_h), s12 = 0.0 - dta * (j1[1] * one_by_h);
+    const double s21 = 0.0 - dta * (j2[0] * one_by_h), s22 = org[2] - dta * (j2[1] * one_by_h);
     const double inv_det = ddiv64(1.0, s11 * s22 - s21 * s12);
+    double nrm = 0.0;
 #pragma unroll
     for (int i = 0; i < nv; ++i) {
       // explicit rows: diagonal org, no coupling into the implicit rows
-      if (i != 1 && i != 2) p[i] = d64_zero(f[i]) ? 0.0 : -ddiv64(f[i], org[i]);
+      if (i == 1) p[1] = -((f[1] * s22 - f[2] * s12) * inv_det) + 0.0;
+      else if (i == 2) p[2] = -((s11 * f[2] - s21 * f[1]) * inv_det) + 0.0;
+      else p[i] = d64_zero(f[i]) ? 0.0 : -ddiv64(f[i], org[i]);
       xo[i] = rel[i];
+      nrm += p[i] * p[i];
     }
-    p[1] = -((f[1] * s22 - f[2] * s12) * inv_det) + 0.0;
-    p[2] = -((s11 * f[2] - s21 * f[1]) * inv_det) + 0.0;
-    const double scal_old = scal_f;
-    if (it == 1) {
-#pragma unroll
-      for (int i = 0; i < nv; ++i) {
-        rel[i] = xo[i] + p[i];
-        qj[i] = rel[i] * org[i];
-      }
-      friction_real<NS>(P, c.Bx, c.By, dxi, qj, fp, nh1, nh2);
-      newton_residual<NS>(c, dtR, qj, nh1, nh2, f, scal_f);
-    } else {
-      double nrm = 0.0;
-#pragma unroll
-      for (int i = 0; i < nv; ++i) nrm += p[i] * p[i];
-      // gradient of the old residual (explicit columns: diagonal org)
-      double g[nv];
-#pragma unroll
-      for (int i = 0; i < nv; ++i) g[i] = f[i];
+    scal_old = scal_f;
+    phase = (it == 1) ? FIRST : TRIAL;
+    if (it > 1) {
+      alam = 1.0;
+      slope = 0.0;
+      alamin = -1.0;
       if (!d64_lt(nrm, (99.0 * nv) * (99.0 * nv))) {
         // |p| may pass the largest step, 100 max(|x|, n_vars)
         nrm = sqrt(nrm);
@@ -348,103 +383,32 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
 #pragma unroll
           for (int i = 0; i < nv; ++i) p[i] = p[i] * stpmax / nrm;
         }
-      }
-      bool huge = false;
-#pragma unroll
-      for (int i = 0; i < nv; ++i) huge = huge || (d64_hi(fabs(p[i])) >= 0x7e000000);   // TOLX / max |p| may be 0
-      double alam = 1.0, alam2 = 0.0, f2 = 0.0, tmplam = 0.0, slope = 0.0, alamin = -1.0;
-      check = false;
-      for (int ls = 0; ls < 4096; ++ls) {
-        if (alamin < 0.0 && (ls > 0 || huge)) {
-          slope = 0.0;
-          double mx = 0.0;
-#pragma unroll
-          for (int i = 0; i < nv; ++i) {
-            const double gi = (i == 1) ? g[1] * s11 + g[2] * s21 : (i == 2) ? g[1] * s12 + g[2] * s22 : g[i] * org[i];
-            slope += gi * p[i];
-            const double ax = fabs(xo[i]), t = fabs(p[i]) / (ax > 1.0 ? ax : 1.0);
-            if (i == 0 || t > mx) mx = t;
-          }
-          alamin = TOLX / mx;
-          if (alamin == 0.0) {   // only before the first trial
-#pragma unroll
-            for (int i = 0; i < nv; ++i) rel[i] = xo[i];
-            break;
-          }
-        }
-        if (ls > 0) {
-          // the last trial was refused
-          if (alam < alamin) {
-#pragma unroll
-            for (int i = 0; i < nv; ++i) rel[i] = xo[i];
-            scal_f = scal_old;
-            check = true;
-            break;
-          }
-          if (alam == 1.0) {
-            tmplam = -slope / (2.0 * (scal_f - scal_old - slope));
-          } else {
-            const double rhs1 = scal_f - scal_old - alam * slope;
-            const double rhs2 = f2 - scal_old - alam2 * slope;
-            const double a = (rhs1 / (alam * alam) - rhs2 / (alam2 * alam2)) / (alam - alam2);
-            const double b = (-alam2 * rhs1 / (alam * alam) + alam * rhs2 / (alam2 * alam2)) / (alam - alam2);
-            if (a == 0.0) {
-              tmplam = -slope / (2.0 * b);
-            } else {
-              const double disc = b * b - 3.0 * a * slope;
-              if (disc < 0.0) tmplam = 0.5 * alam;
-              else if (b <= 0.0) tmplam = (-b + sqrt(disc)) / (3.0 * a);
-              else tmplam = -slope / (b + sqrt(disc));
-            }
-            if (tmplam > 0.5 * alam) tmplam = 0.5 * alam;
-          }
-          alam2 = alam;
-          f2 = scal_f;
-          alam = (tmplam > 0.5 * alam) ? tmplam : 0.5 * alam;
-        }
+        // a direction so long that TOLX / max |p| is 0 is not tried
+        double mx = 0.0;
 #pragma unroll
         for (int i = 0; i < nv; ++i) {
-          rel[i] = xo[i] + ((ls == 0) ? p[i] : alam * p[i]);
-          qj[i] = rel[i] * org[i];
+          const double ax = fabs(xo[i]), t = fabs(p[i]) / (ax > 1.0 ? ax : 1.0);
+          if (i == 0 || t > mx) mx = t;
         }
-        friction_real<NS>(P, c.Bx, c.By, dxi, qj, fp, nh1, nh2);
-        newton_residual<NS>(c, dtR, qj, nh1, nh2, f, scal_f);
-        if (!d64_lt(0.9 * scal_old, scal_f) && (d64_bits(scal_f) & kD64Abs) <= kD64Inf) break;
-      }
-      if (check) {
-        // the convergence test on the gradient at the restored point
-        double mc = 0.0;
+        alamin = TOLX / mx;
+        if (alamin == 0.0) {
 #pragma unroll
-        for (int i = 0; i < nv; ++i) {
-          const double gi = (i == 1) ? g[1] * s11 + g[2] * s21 : (i == 2) ? g[1] * s12 + g[2] * s22 : g[i] * org[i];
-          const double ar = fabs(rel[i]), m = (ar > 1.0 ? ar : 1.0), d = (scal_f > 0.5 * nv) ? scal_f : 0.5 * nv;
-          const double t = fabs(gi) * m / d;
-          mc = (mc > t) ? mc : t;
+          for (int i = 0; i < nv; ++i) qj[i] = xo[i] * org[i];
+          return it;
         }
-        check = mc < TOLMIN;
       }
+      // derivative of the half square sum along p (explicit columns of the
+      // matrix: diagonal org)
+#pragma unroll
+      for (int i = 0; i < nv; ++i)
+        slope += ((i == 1) ? f[1] * s11 + f[2] * s21 : (i == 2) ? f[1] * s12 + f[2] * s22 : f[i] * org[i]) * p[i];
     }
-#pragma unroll
-    for (int i = 0; i < nv; ++i) qj[i] = rel[i] * org[i];
-    if (newton_maxf<NS>(f) < d64_bits(TOLF)) return it;
-    // |step| < TOLX max(|rel|, 1) in every component: TOLX is a power of
-    // two, so the product is exact and orders as the quotient does
-    // (a NaN component is forgotten when a later one is a number, as the
-    // maximum forgets it)
-    bool small = true, was_nan = false;
 #pragma unroll
     for (int i = 0; i < nv; ++i) {
-      const double ar = fabs(rel[i]), st = fabs(rel[i] - xo[i]);
-      small = (small || was_nan) && d64_lt(st, TOLX * (d64_lt(1.0, ar) ? ar : 1.0));
-      was_nan = d64_bits(st) > kD64Inf || (d64_bits(st) == kD64Inf && d64_bits(ar) == kD64Inf);
-    }
-    if (small) return it;
-    if (!isfinite(scal_f)) {
-      // the next iteration's first tests: not converged, not finite
-      return kMaxNewton + 1;
+      rel[i] = xo[i] + p[i];
+      qj[i] = rel[i] * org[i];
     }
   }
-  return kMaxNewton + 1;
 }
 
 }  // namespace sflow

@@ -630,9 +630,10 @@ __device__ __forceinline__ bool rel_below(R d, R s, R tol) {
   return rdiv<R>(d, s) < tol;
 }
 
+// (the FP64 form calls one copy for all classes: instruction cache)
 template <class R>
-__device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos, R rhoc,
-                                               R inv_kin_visc) {
+__device__ __forceinline__ R settling_velocity_inl(const Phys<R>& P, R diam, R rhos, R rhoc,
+                                                   R inv_kin_visc) {
   R inv_sqrt_C_D = R(1);
   if (rhos <= rhoc) return R(0);
   R const_part = rroot<R>((cst<R>(4.0) / cst<R>(3.0)) * (rdiv<R>(rhos, rhoc) - R(1)) * diam * P.grav);
@@ -652,6 +653,16 @@ __device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos,
     }
   }
   return sv;
+}
+
+static __device__ __noinline__ double settling_velocity64(const Phys<double>& P, double diam, double rhos, double rhoc,
+                                                          double inv_kin_visc) {
+  return settling_velocity_inl<double>(P, diam, rhos, rhoc, inv_kin_visc);
+}
+template <class R>
+__device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos, R rhoc, R inv_kin_visc) {
+  if constexpr (sizeof(R) == 8) return settling_velocity64(P, diam, rhos, rhoc, inv_kin_visc);
+  else return settling_velocity_inl<R>(P, diam, rhos, rhoc, inv_kin_visc);
 }
 
 // erodible: the cell's erodible solid thicknesses (null: none, as with

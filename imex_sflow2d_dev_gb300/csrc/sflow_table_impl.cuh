@@ -120,8 +120,11 @@ __global__ void k_stats_partial(KArgs<R> a, double* __restrict__ part) {
 
 
 // ---- tile-height dependent entries (one translation unit per height) ----
-// pointwise kernels of a single run: one block per 32 x 8 cells
-static inline dim3 stage_grid(dim3 tiles, int ny) { return dim3(tiles.x, (unsigned)((ny + 7) / 8)); }
+// pointwise kernels of a single run: one block per 32 x ROWS cells
+template <class R>
+static inline dim3 stage_grid(dim3 tiles, int ny) {
+  return dim3(tiles.x, (unsigned)((ny + StageShape<R>::ROWS - 1) / StageShape<R>::ROWS));
+}
 
 template <class R, int NS, int TH>
 static cudaError_t tab_mask(const KArgs<R>& a, dim3 grid, cudaStream_t s, int solve_all) {
@@ -138,17 +141,17 @@ static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStrea
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_stage2(const KArgs<R>& a, dim3 grid, cudaStream_t s, int mode) {
-  return launch_step_kernel(k_stage2<R, NS, TH>, stage_grid(grid, a.g.ny), dim3(TileShape<TH>::STAGE_THREADS), 0, s,
+  return launch_step_kernel(k_stage2<R, NS, TH>, stage_grid<R>(grid, a.g.ny), dim3(StageShape<R>::THREADS), 0, s,
                             a.g.pdl, a, mode);
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_stage(const KArgs<R>& a, dim3 grid, cudaStream_t s, int irk) {
-  return launch_step_kernel(k_stage<R, NS, TH>, stage_grid(grid, a.g.ny), dim3(TileShape<TH>::STAGE_THREADS), 0, s,
+  return launch_step_kernel(k_stage<R, NS, TH>, stage_grid<R>(grid, a.g.ny), dim3(StageShape<R>::THREADS), 0, s,
                             a.g.pdl, a, irk);
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_assemble(const KArgs<R>& a, dim3 grid, cudaStream_t s) {
-  return launch_step_kernel(k_assemble<R, NS, TH>, stage_grid(grid, a.g.ny), dim3(TileShape<TH>::STAGE_THREADS), 0,
+  return launch_step_kernel(k_assemble<R, NS, TH>, stage_grid<R>(grid, a.g.ny), dim3(StageShape<R>::THREADS), 0,
                             s, a.g.pdl, a);
 }
 template <class R, int NS, int TH>
@@ -174,7 +177,7 @@ static cudaError_t tab_b_setup(size_t smem_flux, int* grids) {
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_b_flux<R, NS, -1, TH>, TileShape<TH>::FLUX_THREADS,
                                                     smem_flux);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], k_b_stage2<R, NS, TH>, kBatchStageThreads, 0);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], k_b_stage2<R, NS, TH>, kBatchStageThreads<R>, 0);
   if (e != cudaSuccess) return e;
   grids[0] = sms * 4;
   grids[1] = sms * (occ[0] > 0 ? occ[0] : 1);
@@ -201,7 +204,7 @@ static cudaError_t tab_b_step(const BatchArgs<R>& b, cudaStream_t s, const int* 
   if (e == cudaSuccess) e = launch_step_kernel(k_b_dt<R>, dim3(1), dim3(kBatchCandThreads), 0, s, pdl, b);
   if (e == cudaSuccess) e = rec(4);
   if (e == cudaSuccess)
-    e = launch_step_kernel(k_b_stage2<R, NS, TH>, dim3(grids[3]), dim3(kBatchStageThreads), 0, s, pdl, b);
+    e = launch_step_kernel(k_b_stage2<R, NS, TH>, dim3(grids[3]), dim3(kBatchStageThreads<R>), 0, s, pdl, b);
   if (e == cudaSuccess) e = rec(5);
   return e;
 }
