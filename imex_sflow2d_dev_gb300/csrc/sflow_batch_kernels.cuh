@@ -43,6 +43,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "sflow_flux64.cuh"
 #include "sflow_kernels.cuh"
 
 namespace sflow {
@@ -340,6 +341,38 @@ __global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, TileShape<TH>::FL
   }
 }
 
+// The FP64 form: items are 4, 2 or 1 rows of a tile, the most that still give
+// every block one (see flux64_rows).
+template <int NS, int LIM>
+__global__ void __launch_bounds__(kFlux64Threads, 3) k_b_flux64(BatchArgs<double> b) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ __align__(16) unsigned char sa_raw[sizeof(KArgs<double>)];
+  __shared__ unsigned s_idx[2];
+  step_kernel_entry();
+  KArgs<double>& a = *reinterpret_cast<KArgs<double>*>(sa_raw);
+  BatchCtl* ctl = b.ctl;
+  const unsigned pp = ctl->pp;
+  const unsigned long long* L = pp ? b.list0 : b.list1;
+  const unsigned n = ctl->count[pp ^ 1u];
+  const unsigned parts = n * 2u >= gridDim.x ? 2u : (n * 4u >= gridDim.x ? 4u : 8u);
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->work[2] = 0u;
+  int cur = -1;
+  TileQueue tq{&ctl->work[1], s_idx};
+  for (unsigned i = tq.first(); i < n * parts; i = tq.next()) {
+    tq.prefetch();
+    const unsigned long long e = L[i / parts];
+    const int slot = entry_slot(e);
+    const unsigned tile = entry_tile(e);
+    if (slot != cur) {
+      load_args(&a, &b.args[slot]);
+      cur = slot;
+      __syncthreads();
+    }
+    const int tiles_x = (a.g.nx + TX - 1) / TX;
+    flux_tile64<NS, LIM>(a, a.q, a.rd, 1, (int)(tile % (unsigned)tiles_x), (int)(tile / (unsigned)tiles_x),
+                         (int)(i % parts * (8u / parts)), (int)(8u / parts), smem_raw);
+  }
+}
 
 template <class R>
 __global__ void __launch_bounds__(kBatchCandThreads) k_b_dt(BatchArgs<R> b) {

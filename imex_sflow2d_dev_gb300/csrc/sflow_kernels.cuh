@@ -746,7 +746,7 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
   constexpr int nv = 4 + NS, ns = NS;
   R a1 = rmin(rmin(L.vmin, Rt.vmin), R(0));
   R a2 = rmax(rmax(L.vmax, Rt.vmax), R(0));
-  if (a1 == a2) {
+  if (sizeof(R) == 8 ? iszero<R>(a1) && iszero<R>(a2) : a1 == a2) {   // a1 <= 0 <= a2
 #pragma unroll
     for (int i = 0; i < nv; ++i) H[i] = R(0);
   } else {
@@ -777,7 +777,8 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
         for (int i = 0; i < ns; ++i) s2 += H[4 + i];
         // s2 / H[0] >= 1 without the quotient: rounded, it reaches 1 exactly
         // when s2 reaches H[0] (the next number below lies more than 2^-54 away)
-        const bool over = H[0] > R(0) ? s2 >= H[0] : (H[0] < R(0) ? s2 <= H[0] : s2 / H[0] >= R(1));
+        const bool over = ispos<R>(H[0]) ? !rlt<R>(s2, H[0]) && s2 == s2
+                                         : (isneg<R>(H[0]) ? !rlt<R>(H[0], s2) && s2 == s2 : s2 / H[0] >= R(1));
         s2 = over ? R(1) : R(0);
         if (over) {
 #pragma unroll
@@ -791,16 +792,19 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
     } else {
       R s = R(0);
 #pragma unroll
-      for (int i = 0; i < ns; ++i) s += H[4 + i];
-      const R r = rdiv<R>(s, H[0]);
-      if (r > R(1)) {
+      for (int i = 0; i < ns; ++i) s = psum<R>(s, H[4 + i], i);
+      bool over;
+      if constexpr (sizeof(R) == 8) over = ispos<R>(H[0]) ? rlt<R>(H[0], s) : (isneg<R>(H[0]) ? rlt<R>(s, H[0]) : s / H[0] > R(1));
+      else over = s / H[0] > R(1);   // FP64: the same without the quotient, as above
+      if (over) {
+        const R r = rdiv<R>(s, H[0]);
 #pragma unroll
         for (int i = 0; i < ns; ++i) H[4 + i] = rdiv<R>(H[4 + i], r);
       }
     }
   }
-  const bool zero_vel = (DIR == 1) ? (L.hu_p == R(0) && Rt.hu_p == R(0))
-                                   : (L.q[2] == R(0) && Rt.q[2] == R(0));
+  const bool zero_vel = (DIR == 1) ? (iszero<R>(L.hu_p) && iszero<R>(Rt.hu_p))
+                                   : (iszero<R>(L.q[2]) && iszero<R>(Rt.q[2]));
   if (zero_vel) {
     H[0] = R(0);
 #pragma unroll

@@ -129,7 +129,7 @@ __device__ __forceinline__ void friction_real(const Phys<double>& P, double Bx, 
     const Div64 dxc = div64(f.xc);
     double T;
     if (!f.film) {
-      const double cp_c = quot64(f.xc * P.sp_heat_a + 0.0, dxc);
+      const double cp_c = quot64(f.xc * P.sp_heat_a, dxc);
       const double cmix = dcp + f.xc * cp_c;
       const double e = P.energy ? q[3] - 0.5 * (q[1] * q[1] + q[2] * q[2]) * f.inv : q[3];
       if (P.energy) {
@@ -141,7 +141,7 @@ __device__ __forceinline__ void friction_real(const Phys<double>& P, double Bx, 
       f.t_amb = T <= 0.0;
     }
     if (f.t_amb) T = P.T_ambient;
-    f.Rc = quot64(f.xc * P.sp_gas_const_a + 0.0, dxc);
+    f.Rc = quot64(f.xc * P.sp_gas_const_a, dxc);
     inv_rho_c = f.Rc * T * P.inv_pres;
   } else {
     inv_rho_c = P.inv_rho_l;   // the temperature does not enter

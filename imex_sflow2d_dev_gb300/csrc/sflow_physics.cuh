@@ -25,10 +25,44 @@ constexpr double kEps = DBL_EPSILON;  // EPSILON(1.0_wp)
 template <class R>
 __device__ __forceinline__ R cst(double x) { return static_cast<R>(x); }
 
+// a < b, x > t (t a positive constant), x > 0, x < 0, x == 0: the FP64 form's
+// on the integer pipes with the same answers (sflow_div64.cuh)
 template <class R>
-__device__ __forceinline__ R rmin(R a, R b) { return a < b ? a : b; }
+__device__ __forceinline__ bool rlt(R a, R b) {
+  if constexpr (sizeof(R) == 8) return d64_lt(a, b);
+  else return a < b;
+}
 template <class R>
-__device__ __forceinline__ R rmax(R a, R b) { return a > b ? a : b; }
+__device__ __forceinline__ bool above(R x, R t) {
+  if constexpr (sizeof(R) == 8) return d64_gt_pos(x, t);
+  else return x > t;
+}
+template <class R>
+__device__ __forceinline__ bool ispos(R x) {
+  if constexpr (sizeof(R) == 8) return d64_pos(x);
+  else return x > R(0);
+}
+template <class R>
+__device__ __forceinline__ bool isneg(R x) {
+  if constexpr (sizeof(R) == 8) return d64_neg(x);
+  else return x < R(0);
+}
+template <class R>
+__device__ __forceinline__ bool iszero(R x) {
+  if constexpr (sizeof(R) == 8) return d64_zero(x);
+  else return x == R(0);
+}
+template <class R>
+__device__ __forceinline__ R rmin(R a, R b) { return rlt<R>(a, b) ? a : b; }
+template <class R>
+__device__ __forceinline__ R rmax(R a, R b) { return rlt<R>(b, a) ? a : b; }
+// i-th partial sum of s = 0 + x_0 + x_1 ...: the FP64 form leaves the leading
+// 0 out (a sum of -0 alone would be +0; no closure distinguishes the two)
+template <class R>
+__device__ __forceinline__ R psum(R s, R x, int i) {
+  if constexpr (sizeof(R) == 8) return i == 0 ? x : s + x;
+  else return s + x;
+}
 template <class R>
 __device__ __forceinline__ R sq(R a) { return a * a; }
 // x^y and log x: in the FP64 form the library's own functions (sflow_math.h;
@@ -169,10 +203,10 @@ __device__ __forceinline__ R qc_to_qp(const Phys<R>& P, const R* q, R* qp) {
   constexpr int ns = NS, nv = 4 + NS;
   R xs[kMaxSolid];
   R inv_qj1;
-  if (q[0] > P.thr_eps) {
+  if (above<R>(q[0], P.thr_eps)) {
     inv_qj1 = fdiv(R(1), q[0]);
     R sq_ = R(0);
-    for (int i = 0; i < ns; ++i) { xs[i] = q[4 + i] * inv_qj1; sq_ += q[4 + i]; }
+    for (int i = 0; i < ns; ++i) { xs[i] = q[4 + i] * inv_qj1; sq_ = psum<R>(sq_, q[4 + i], i); }
     if (sq_ == q[0]) {
       R s = R(0);
       for (int i = 0; i < ns; ++i) s += xs[i];
@@ -184,14 +218,16 @@ __device__ __forceinline__ R qc_to_qp(const Phys<R>& P, const R* q, R* qp) {
     return R(0);
   }
   R xs_tot = R(0);
-  for (int i = 0; i < ns; ++i) xs_tot += xs[i];
+  for (int i = 0; i < ns; ++i) xs_tot = psum<R>(xs_tot, xs[i], i);
   R xc = R(1) - xs_tot;
-  R cbyxc = P.gas ? ((xc - R(0)) * P.sp_heat_a + R(0)) : P.sp_heat_l * xc;
+  R cbyxc;
+  if constexpr (sizeof(R) == 8) cbyxc = P.gas ? xc * P.sp_heat_a : P.sp_heat_l * xc;
+  else cbyxc = P.gas ? ((xc - R(0)) * P.sp_heat_a + R(0)) : P.sp_heat_l * xc;
   R dcp = R(0);
-  for (int i = 0; i < ns; ++i) dcp += xs[i] * P.sp_heat_s[i];
+  for (int i = 0; i < ns; ++i) dcp = psum<R>(dcp, xs[i] * P.sp_heat_s[i], i);
   R cmix = dcp + cbyxc;
   R T;
-  if (q[0] > P.thr_eps_sing) {
+  if (above<R>(q[0], P.thr_eps_sing)) {
     if (P.energy) T = fdiv(q[3] - cst<R>(0.5) * (sq(q[1]) + sq(q[2])) * inv_qj1, q[0] * cmix);
     else T = fdiv(q[3], q[0] * cmix);
     if (T <= R(0)) T = P.T_ambient;
@@ -204,18 +240,18 @@ __device__ __forceinline__ R qc_to_qp(const Phys<R>& P, const R* q, R* qp) {
     // as such; the FP64 form keeps the reference's operations)
     R Rc;
     if constexpr (sizeof(R) == 4) Rc = P.sp_gas_const_a;
-    else Rc = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_gas_const_a + R(0), xc) : P.sp_gas_const_a;
+    else Rc = above<R>(xc, P.thr_eps) ? rdiv<R>(xc * P.sp_gas_const_a, xc) : P.sp_gas_const_a;
     inv_rho_c = Rc * T * P.inv_pres;
   } else {
     inv_rho_c = P.inv_rho_l;
   }
   R dinv = R(0);
-  for (int i = 0; i < ns; ++i) dinv += xs[i] * P.inv_rho_s[i];
+  for (int i = 0; i < ns; ++i) dinv = psum<R>(dinv, xs[i] * P.inv_rho_s[i], i);
   R inv_rhom = dinv + xc * inv_rho_c;
   R rho_m = fdiv(R(1), inv_rhom);
   R h = q[0] * inv_rhom;
   R u, v;
-  if (q[0] > P.thr_eps_sing) {
+  if (above<R>(q[0], P.thr_eps_sing)) {
     u = q[1] * inv_qj1;
     v = q[2] * inv_qj1;
   } else {
@@ -268,7 +304,7 @@ __device__ __forceinline__ void qp_to_qc(const Phys<R>& P, const R* qp, R* qc) {
     R rho_a = fdiv(P.pres, P.sp_gas_const_a * r_T);
     // carrier of air alone: ((1 - at) rho_a) / (1 - at) is rho_a
     if constexpr (sizeof(R) == 4) rho_c = rho_a;
-    else rho_c = rdiv<R>((R(1) - R(0) - at - R(0)) * rho_a + R(0), R(1) - R(0) - at);
+    else rho_c = rdiv<R>((R(1) - at) * rho_a, R(1) - at);
   } else {
     rho_c = P.rho_l;
   }
@@ -281,7 +317,7 @@ __device__ __forceinline__ void qp_to_qc(const Phys<R>& P, const R* qp, R* qc) {
   R cp_c;
   if (P.gas) {
     if constexpr (sizeof(R) == 4) cp_c = P.sp_heat_a;   // (x_c c_a) / x_c
-    else cp_c = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_heat_a + R(0), xc) : P.sp_heat_a;
+    else cp_c = above<R>(xc, P.thr_eps) ? rdiv<R>(xc * P.sp_heat_a, xc) : P.sp_heat_a;
   } else {
     cp_c = P.sp_heat_l;
   }
@@ -310,7 +346,7 @@ __device__ __forceinline__ Mixt<R> mixt_var(const Phys<R>& P, const R* qpj, bool
   constexpr int ns = NS, nv = 4 + NS;
   Mixt<R> m;
   R r_h = qpj[0];
-  if (!(qpj[0] > P.thr_eps)) {
+  if (!above<R>(qpj[0], P.thr_eps)) {
     m.red_grav = R(0); m.rho_m = P.rho_a_amb; m.rho_c = P.rho_a_amb;
     m.cp_c = P.liquid ? P.sp_heat_l : P.sp_heat_a;
     m.cp_mix = m.cp_c;
@@ -320,18 +356,18 @@ __device__ __forceinline__ Mixt<R> mixt_var(const Phys<R>& P, const R* qpj, bool
   R r_u = qpj[nv], r_v = qpj[nv + 1], r_T = qpj[3];
   R al[kMaxSolid];
   R at = R(0);
-  for (int i = 0; i < ns; ++i) { al[i] = P.alpha ? qpj[4 + i] : fdiv(qpj[4 + i], qpj[0]); at += al[i]; }
+  for (int i = 0; i < ns; ++i) { al[i] = P.alpha ? qpj[4 + i] : fdiv(qpj[4 + i], qpj[0]); at = psum<R>(at, al[i], i); }
   R rho_c;
   if (P.gas) {
     R rho_a = fdiv(P.pres, P.sp_gas_const_a * r_T);
     // carrier of air alone: ((1 - at) rho_a) / (1 - at) is rho_a
     if constexpr (sizeof(R) == 4) rho_c = rho_a;
-    else rho_c = rdiv<R>((R(1) - R(0) - at - R(0)) * rho_a + R(0), R(1) - R(0) - at);
+    else rho_c = rdiv<R>((R(1) - at) * rho_a, R(1) - at);
   } else {
     rho_c = P.rho_l;
   }
   R d = R(0);
-  for (int i = 0; i < ns; ++i) d += al[i] * P.rho_s[i];
+  for (int i = 0; i < ns; ++i) d = psum<R>(d, al[i] * P.rho_s[i], i);
   R rho_m = (R(1) - at) * rho_c + d;
   R inv_rhom, red_grav;
   if constexpr (sizeof(R) == 4) {
@@ -343,7 +379,7 @@ __device__ __forceinline__ Mixt<R> mixt_var(const Phys<R>& P, const R* qpj, bool
     red_grav = quot64(rho_m - P.rho_a_amb, vm) * P.grav;
   }
   R u2 = sq(r_u) + sq(r_v);
-  m.Ri = (u2 > R(0)) ? rmin(cst<R>(1.0e15), fdiv(red_grav * r_h, u2)) : R(0);
+  m.Ri = ispos<R>(u2) ? rmin(cst<R>(1.0e15), fdiv(red_grav * r_h, u2)) : R(0);
   m.rho_m = rho_m;
   m.rho_c = rho_c;
   m.red_grav = red_grav;
@@ -352,17 +388,17 @@ __device__ __forceinline__ Mixt<R> mixt_var(const Phys<R>& P, const R* qpj, bool
   if (sp_heat_flag) {
     R xs[kMaxSolid];
     R sxs = R(0);
-    for (int i = 0; i < ns; ++i) { xs[i] = al[i] * P.rho_s[i] * inv_rhom; sxs += xs[i]; }
+    for (int i = 0; i < ns; ++i) { xs[i] = al[i] * P.rho_s[i] * inv_rhom; sxs = psum<R>(sxs, xs[i], i); }
     R xc = R(1) - sxs;
     R cp_c;
     if (P.gas) {
       if constexpr (sizeof(R) == 4) cp_c = P.sp_heat_a;   // (x_c c_a) / x_c
-      else cp_c = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_heat_a + R(0), xc) : P.sp_heat_a;
+      else cp_c = above<R>(xc, P.thr_eps) ? rdiv<R>(xc * P.sp_heat_a, xc) : P.sp_heat_a;
     } else {
       cp_c = P.sp_heat_l;
     }
     R dcp = R(0);
-    for (int i = 0; i < ns; ++i) dcp += xs[i] * P.sp_heat_s[i];
+    for (int i = 0; i < ns; ++i) dcp = psum<R>(dcp, xs[i] * P.sp_heat_s[i], i);
     m.cp_c = cp_c;
     m.cp_mix = dcp + xc * cp_c;
   }
@@ -381,7 +417,7 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
   m.cp_c = R(0);
   m.cp_mix = R(0);
   R r_h = qp[0];
-  if (!(r_h > P.thr_eps)) {
+  if (!above<R>(r_h, P.thr_eps)) {
     for (int i = 0; i < nv; ++i) qc[i] = R(0);
     m.red_grav = R(0); m.rho_m = P.rho_a_amb; m.rho_c = P.rho_a_amb;
     return m;
@@ -391,7 +427,7 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
   R at = R(0);
   for (int i = 0; i < ns; ++i) {
     R al = P.alpha ? qp[4 + i] : fdiv(qp[4 + i], qp[0]);
-    at += al;
+    at = psum<R>(at, al, i);
     arhos[i] = al * P.rho_s[i];
   }
   R rho_c;
@@ -399,13 +435,13 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
     R rho_a = fdiv(P.pres, P.sp_gas_const_a * r_T);
     // carrier of air alone: ((1 - at) rho_a) / (1 - at) is rho_a
     if constexpr (sizeof(R) == 4) rho_c = rho_a;
-    else rho_c = rdiv<R>((R(1) - R(0) - at - R(0)) * rho_a + R(0), R(1) - R(0) - at);
+    else rho_c = rdiv<R>((R(1) - at) * rho_a, R(1) - at);
   } else {
     rho_c = P.rho_l;
   }
   R alphac = R(1) - at;
   R sa = R(0);
-  for (int i = 0; i < ns; ++i) sa += arhos[i];
+  for (int i = 0; i < ns; ++i) sa = psum<R>(sa, arhos[i], i);
   R rho_m = alphac * rho_c + sa;
   R inv_rhom;
   if constexpr (sizeof(R) == 4) {
@@ -419,18 +455,18 @@ __device__ __forceinline__ Mixt<R> qp_to_qc_mixt(const Phys<R>& P, const R* qp, 
   R cp_c;
   if (P.gas) {
     if constexpr (sizeof(R) == 4) cp_c = P.sp_heat_a;   // (x_c c_a) / x_c
-    else cp_c = (xc > P.thr_eps) ? rdiv<R>((xc - R(0)) * P.sp_heat_a + R(0), xc) : P.sp_heat_a;
+    else cp_c = above<R>(xc, P.thr_eps) ? rdiv<R>(xc * P.sp_heat_a, xc) : P.sp_heat_a;
   } else {
     cp_c = P.sp_heat_l;
   }
   R dcp = R(0);
-  for (int i = 0; i < ns; ++i) dcp += (arhos[i] * inv_rhom) * P.sp_heat_s[i];
+  for (int i = 0; i < ns; ++i) dcp = psum<R>(dcp, (arhos[i] * inv_rhom) * P.sp_heat_s[i], i);
   R cmix = dcp + xc * cp_c;
   qc[0] = rho_m * r_h;
   qc[1] = rho_m * r_hu;
   qc[2] = rho_m * r_hv;
   if (P.energy) {
-    qc[3] = (r_h > R(0)) ? r_h * rho_m * (cmix * r_T + cst<R>(0.5) * (sq(r_u) + sq(r_v))) : R(0);
+    qc[3] = ispos<R>(r_h) ? r_h * rho_m * (cmix * r_T + cst<R>(0.5) * (sq(r_u) + sq(r_v))) : R(0);
   } else {
     qc[3] = r_h * rho_m * cmix * r_T;
   }
@@ -448,7 +484,7 @@ __device__ __forceinline__ void local_speeds(const Phys<R>& P, const R* qpj, R r
   constexpr int nv = 4 + NS;
   R r_h = qpj[0];
   R vel = (dir == 1) ? qpj[nv] : qpj[nv + 1];
-  if (red_grav * r_h < R(0)) {
+  if (isneg<R>(red_grav * r_h)) {
     vmin = vel; vmax = vel;
   } else {
     R c = (dir == 1) ? rroot<R>(red_grav * r_h * gc) : rroot<R>(gc * red_grav * r_h);
@@ -462,7 +498,7 @@ template <class R, int NS>
 __device__ __forceinline__ void eval_fluxes(const Phys<R>& P, const R* qcj, const R* qpj,
                                             const Mixt<R>& m, R gc, int dir, R* flux) {
   constexpr int ns = NS, nv = 4 + NS;
-  if (qpj[0] > P.thr_eps) {
+  if (above<R>(qpj[0], P.thr_eps)) {
     R r_h = qpj[0];
     R vel = (dir == 1) ? qpj[nv] : qpj[nv + 1];
     R pterm = cst<R>(0.5) * m.rho_m * gc * m.red_grav * sq(r_h);
@@ -476,12 +512,12 @@ __device__ __forceinline__ void eval_fluxes(const Phys<R>& P, const R* qcj, cons
     }
     flux[3] = P.energy ? vel * (qcj[3] * R(1) + pterm) : vel * qcj[3] * R(1);
     for (int i = 0; i < ns; ++i) flux[4 + i] = vel * qcj[4 + i] * R(1);
-    if (ns > 0 && flux[0] > R(0)) {
+    if (ns > 0 && ispos<R>(flux[0])) {
       R s = R(0);
-      for (int i = 0; i < ns; ++i) s += flux[4 + i];
+      for (int i = 0; i < ns; ++i) s = psum<R>(s, flux[4 + i], i);
       // flux[0] > 0 here: s / flux[0], rounded, is above 1 exactly when s is
       // above flux[0] (the next number above lies more than 2^-53 away)
-      if (s > flux[0])
+      if (rlt<R>(flux[0], s))
         for (int i = 0; i < ns; ++i) flux[4 + i] = rdiv<R>(flux[4 + i], s) * flux[0];
     }
   } else {
@@ -500,17 +536,18 @@ __device__ __forceinline__ void expl_terms(const Phys<R>& P, const Geo<R>& g, co
                                            R bf, R b_coeff, R b_vel, R* e) {
   constexpr int ns = NS, nv = 4 + NS;
   for (int i = 0; i < nv; ++i) e[i] = R(0);
-  if (!(qpj[0] > P.thr_eps) && bf == R(0) && arc_perim == R(0)) return;
-  if (qpj[0] > P.thr_eps) {
+  const bool wet = above<R>(qpj[0], P.thr_eps);
+  if (!wet && iszero<R>(bf) && iszero<R>(arc_perim)) return;
+  if (wet) {
     R r_h = qpj[0], r_u = qpj[nv], r_v = qpj[nv + 1];
-    Mixt<R> m = mixt_var<R, NS>(P, qpj, true);
+    Mixt<R> m = mixt_var<R, NS>(P, qpj, sizeof(R) == 4);   // specific heats not read (FP64: not formed)
     R centr = P.curv ? (g.Bxx * sq(r_u) + cst<R>(2.0) * g.Bxy * r_u * r_v + g.Byy * sq(r_v)) : R(0);
     R tg = m.red_grav + centr;
     e[1] = -g.gc * m.rho_m * tg * r_h * g.Bx + cst<R>(0.5) * m.rho_m * m.red_grav * sq(r_h) * g.dgcx;
     e[2] = -g.gc * m.rho_m * tg * r_h * g.By + cst<R>(0.5) * m.rho_m * m.red_grav * sq(r_h) * g.dgcy;
     e[3] = P.energy ? (e[1] * r_u + e[2] * r_v) : R(0);
   }
-  if (P.bottom_source && bf > R(0)) {
+  if (P.bottom_source && ispos<R>(bf)) {
     // inflow state: h = 1, T = T_source, alphas_source (its mixt_var is
     // src_rho_m, src_cp_mix); the momentum terms add zero
     const R h_dot = bf * b_vel;
@@ -520,7 +557,7 @@ __device__ __forceinline__ void expl_terms(const Phys<R>& P, const Geo<R>& g, co
     e[3] = e[3] + b_coeff * h_dot * P.src_rho_m * P.src_cp_mix * P.T_source;
     for (int i = 0; i < ns; ++i) e[4 + i] = e[4 + i] + b_coeff * h_dot * P.alphas_source[i] * P.rho_s[i];
   }
-  if (P.radial_source && arc_perim > R(0) && P.h_source > R(0)) {
+  if (P.radial_source && ispos<R>(arc_perim) && P.h_source > R(0)) {
     R t_coeff = t_coeff_src;
     if (t_coeff > R(0)) {
       R h_dot = rdiv<R>(P.h_source * P.vel_source * arc_perim, P.cell_area);

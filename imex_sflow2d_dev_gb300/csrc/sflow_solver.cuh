@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "sflow_host.h"
+#include "sflow_flux64.cuh"
 #include "sflow_kernels.cuh"
 #include "sflow_table.h"
 
@@ -334,6 +335,7 @@ class Solver : public SolverBase {
   // y-face fluxes and speeds, the tile's 5 topography planes, flag bytes of
   // the tile + halo
   static size_t flux_smem_bytes(int nv, int th) {
+    if constexpr (sizeof(R) == 8) return flux64_smem_bytes(nv);
     const int np = nv + 2;
     const size_t ry = (size_t)th + 2 * HALO;
     const size_t r = (size_t)np * RX * ry + (size_t)nv * th * (TX + 1) + (size_t)nv * (th + 1) * TX +

@@ -2,6 +2,7 @@
 // kernels; included by the sflow_k_*.cu translation units only.
 #pragma once
 #include "sflow_batch_kernels.cuh"
+#include "sflow_flux64.cuh"
 #include "sflow_kernels.cuh"
 #include "sflow_table.h"
 
@@ -119,6 +120,12 @@ __global__ void k_stats_partial(KArgs<R> a, double* __restrict__ part) {
 }
 
 
+static inline cudaError_t sm_count(int* sms) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  return e != cudaSuccess ? e : cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+}
+
 // ---- tile-height dependent entries (one translation unit per height) ----
 // pointwise kernels of a single run: one block per 32 x ROWS cells
 template <class R>
@@ -135,9 +142,20 @@ static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStrea
                             R* rout, int want_dt) {
   // minmod everywhere (the reference default) has its own instantiation:
   // one limiter case instead of eight per variable keeps the code small
-  const dim3 T(TileShape<TH>::FLUX_THREADS);
-  if (a.g.lim_all == 1) return launch_step_kernel(k_flux<R, NS, 1, TH>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt);
-  return launch_step_kernel(k_flux<R, NS, -1, TH>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt);
+  if constexpr (sizeof(R) == 8) {
+    int sms = 0;
+    const cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    const int sh = flux64_rows((int64_t)grid.x * grid.y, sms);
+    grid.y *= 8 / sh;
+    const dim3 T(kFlux64Threads);
+    if (a.g.lim_all == 1) return launch_step_kernel(k_flux64<NS, 1>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt, sh);
+    return launch_step_kernel(k_flux64<NS, -1>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt, sh);
+  } else {
+    const dim3 T(TileShape<TH>::FLUX_THREADS);
+    if (a.g.lim_all == 1) return launch_step_kernel(k_flux<R, NS, 1, TH>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt);
+    return launch_step_kernel(k_flux<R, NS, -1, TH>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt);
+  }
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_stage2(const KArgs<R>& a, dim3 grid, cudaStream_t s, int mode) {
@@ -156,26 +174,38 @@ static cudaError_t tab_assemble(const KArgs<R>& a, dim3 grid, cudaStream_t s) {
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_smem(size_t bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k_flux<R, NS, 1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_flux<R, NS, -1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if constexpr (sizeof(R) == 8) {
+    cudaError_t e = cudaFuncSetAttribute(k_flux64<NS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_flux64<NS, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  } else {
+    cudaError_t e = cudaFuncSetAttribute(k_flux<R, NS, 1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_flux<R, NS, -1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  }
 }
+// the batched flux kernel of a form and its threads
+template <class R, int NS, int LIM, int TH>
+static auto batch_flux_kernel() {
+  if constexpr (sizeof(R) == 8) return &k_b_flux64<NS, LIM>;
+  else return &k_b_flux<R, NS, LIM, TH>;
+}
+template <class R, int TH>
+constexpr int kBatchFluxThreads = sizeof(R) == 8 ? kFlux64Threads : TileShape<TH>::FLUX_THREADS;
 template <class R, int NS, int TH>
 static cudaError_t tab_b_setup(size_t smem_flux, int* grids) {
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  int sms = 0;
+  cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  e = cudaFuncSetAttribute(batch_flux_kernel<R, NS, 1, TH>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_flux);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_b_flux<R, NS, 1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_flux);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_b_flux<R, NS, -1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_flux);
+  e = cudaFuncSetAttribute(batch_flux_kernel<R, NS, -1, TH>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_flux);
   if (e != cudaSuccess) return e;
   int occ[3] = {0, 0, 0};
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_b_mask<R, TH>, TileShape<TH>::MASK_THREADS, 0);
   if (e != cudaSuccess) return e;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_b_flux<R, NS, -1, TH>, TileShape<TH>::FLUX_THREADS,
-                                                    smem_flux);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], batch_flux_kernel<R, NS, -1, TH>(),
+                                                    kBatchFluxThreads<R, TH>, smem_flux);
   if (e != cudaSuccess) return e;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], k_b_stage2<R, NS, TH>, kBatchStageThreads<R>, 0);
   if (e != cudaSuccess) return e;
@@ -188,7 +218,7 @@ static cudaError_t tab_b_setup(size_t smem_flux, int* grids) {
 template <class R, int NS, int TH>
 static cudaError_t tab_b_step(const BatchArgs<R>& b, cudaStream_t s, const int* grids, size_t smem_flux, int lim,
                               int pdl, cudaEvent_t* ev) {
-  const dim3 T(TileShape<TH>::FLUX_THREADS);
+  const dim3 T(kBatchFluxThreads<R, TH>);
   auto rec = [&](int i) -> cudaError_t { return ev ? cudaEventRecord(ev[i], s) : cudaSuccess; };
   cudaError_t e = rec(0);
   if (e == cudaSuccess) e = launch_step_kernel(k_b_cand<R>, dim3(grids[0]), dim3(kBatchCandThreads), 0, s, pdl, b);
@@ -197,8 +227,8 @@ static cudaError_t tab_b_step(const BatchArgs<R>& b, cudaStream_t s, const int* 
     e = launch_step_kernel(k_b_mask<R, TH>, dim3(grids[1]), dim3(TileShape<TH>::MASK_THREADS), 0, s, pdl, b);
   if (e == cudaSuccess) e = rec(2);
   if (e == cudaSuccess) {
-    if (lim == 1) e = launch_step_kernel(k_b_flux<R, NS, 1, TH>, dim3(grids[2]), T, smem_flux, s, pdl, b);
-    else e = launch_step_kernel(k_b_flux<R, NS, -1, TH>, dim3(grids[2]), T, smem_flux, s, pdl, b);
+    if (lim == 1) e = launch_step_kernel(batch_flux_kernel<R, NS, 1, TH>(), dim3(grids[2]), T, smem_flux, s, pdl, b);
+    else e = launch_step_kernel(batch_flux_kernel<R, NS, -1, TH>(), dim3(grids[2]), T, smem_flux, s, pdl, b);
   }
   if (e == cudaSuccess) e = rec(3);
   if (e == cudaSuccess) e = launch_step_kernel(k_b_dt<R>, dim3(1), dim3(kBatchCandThreads), 0, s, pdl, b);
