@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kBatchCandThreads) k_b_cand(BatchArgs<R> b) {
   }
   // dry border strips (code 3) of the last step: one thread per tile.  With
   // no mass in its 3 x 3 neighbourhood the tile keeps its code, mask and
-  // count (see mask_tile_skippable) and is carried to the next dry-border
+  // count (see mask_tiles_to_do) and is carried to the next dry-border
   // list -- not when a neighbour dilates to every neighbour (tile_seed): it
   // is a candidate of this step then and must not be listed twice.  Else it
   // is its own candidate (it holds no mass, so it dilates only as a
@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS, 2048 / TileShape<
     // k_b_cand listed only running runs, and no run's clock moves before k_b_dt
     const int tx = (int)(tile % (unsigned)br.tiles_x), ty = (int)(tile / (unsigned)br.tiles_x);
     int act = 0;
-    const int code = mask_tile<R, TH>(a, 0, tx, ty, br.tiles_x, true, &act);
+    const int code = (a.tile_static[tile] & TILE_SPECIAL) ? mask_tile<R, TH>(a, 0, tx, ty, br.tiles_x, true, &act)
+                                                          : mask_tile_plain<R, TH>(a, tx, ty, br.tiles_x, &act);
     if (code == 1) {
       // the tile into the active list, its active cells into the cell list
       // (one thread per cell of the tile: thread = row * 32 + column), one

@@ -235,6 +235,56 @@ static_assert(MRX <= 64, "a frame row must fit one 64-bit mask");
 // skip it.
 constexpr uint8_t TILE_DRY_BORDER = 3;
 
+// Static bits of a tile (tile_static, host computed): a static seed (border,
+// ring-boundary or bottom-source cell) within n_RK cells; a border, ring or
+// source cell within the 4-cell frame, or a frame that leaves the domain.
+constexpr uint8_t TILE_SEED = 1, TILE_SPECIAL = 2;
+
+// check_solve of a tile without TILE_SPECIAL, n_RK = 2: only cells with mass
+// are seeds, no cell of the frame needs its flags or a bounds test, and a
+// two-cell frame suffices.  About a quarter of mask_tile's instructions, which
+// bound check_solve.  Same mask, code and counts.
+template <class R, int TH>
+__device__ __forceinline__ int mask_tile_plain(const KArgs<R>& a, int tx, int ty, int tiles_x, int* act_out) {
+  constexpr int H = 2;
+  __shared__ unsigned long long srow[TH + 2 * H];   // bit x: mass at column x - H of the tile
+  const Grid<R>& g = a.g;
+  const int lane = threadIdx.x % TX, warp = threadIdx.x / TX;
+  const R* q0 = a.q + cidx(g, tx * TX, ty * TH);
+  // warp w takes frame row w and, the first 2 H, row TH + w; lane x column x
+  // and, the first 2 H, one of the columns -2, -1, 32, 33
+  const int xe = lane < H ? lane - H : TX + lane - H;
+#pragma unroll
+  for (int r = 0; r < (TH + 2 * H + TH - 1) / TH; ++r) {
+    const int y = warp + r * TH;
+    if (y >= TH + 2 * H) break;   // warp-uniform
+    const R* row = q0 + (int64_t)(y - H) * g.pitch;
+    const R v = row[lane], e = lane < 2 * H ? row[xe] : R(0);
+    const unsigned long long b = __ballot_sync(0xffffffffu, v > R(0));
+    const unsigned long long x = __ballot_sync(0xffffffffu, e > R(0));
+    if (lane == 0) srow[y] = (b << H) | (x & 3ull) | ((x >> H & 3ull) << (TX + H));
+  }
+  __syncthreads();
+  const unsigned long long* m = srow + warp + H;   // row of the cell; cell column = bit lane + H
+  const unsigned long long five = m[0] >> lane, three = (m[-1] | m[1]) >> (lane + 1), one = (m[-2] | m[2]) >> (lane + H);
+  const int act = ((five & 31ull) | (three & 7ull) | (one & 1ull)) != 0ull;
+  a.mask[cidx(g, tx * TX + lane, ty * TH + warp)] = (uint8_t)act;
+  if (act_out) *act_out = act;
+  int cnt, code;
+  if (g.whole) {
+    cnt = __syncthreads_count(act);
+    code = cnt > 0 ? 1 : 0;
+  } else {
+    cnt = __syncthreads_count(act && owned_row(g, ty * TH + warp));
+    code = __syncthreads_or(act) ? 1 : 0;
+  }
+  if (threadIdx.x == 0) {
+    a.tile_active[ty * tiles_x + tx] = (uint8_t)code;
+    if (cnt) atomicAdd((unsigned long long*)&a.st->cells_acc[a.st->steps & 1], (unsigned long long)cnt);
+  }
+  return code;
+}
+
 // One warp evaluates one tile: lane x owns frame columns x and 32 + x
 // (x < 8) of every frame row, the seeds of a row become one 64-bit mask by
 // two ballots, and lane x then tests the cells of tile column x row by
@@ -367,26 +417,55 @@ __device__ __forceinline__ int mask_tile(const KArgs<R>& a, int solve_all, int t
 // code, mask and active count while no tile of its 3 x 3 neighbourhood
 // holds mass: its 4-cell frame then stays dry, and its seeds are static.
 // Only its count is added.
-// Threads 0-8 read the nine wet flags together; one barrier shares the
-// result (block-uniform).
+//
+// The tiles t0 .. t0 + ng - 1 (ng <= 8) of a block at once: 16 lanes per
+// tile, nine of which read the neighbourhood's wet flags.  Returns the tiles
+// to evaluate, one bit each, and in bits 8-15 those with TILE_SPECIAL
+// (block-uniform).
 template <class R>
-__device__ __forceinline__ bool mask_tile_skippable(const KArgs<R>& a, int tx, int ty, int tiles_x, int tiles_y) {
-  const int nt = tiles_x * tiles_y, t = ty * tiles_x + tx;
-  const unsigned par = (unsigned)(a.st->steps & 1);
-  int wet = 0;
-  if (threadIdx.x < 9) {
-    const int x = tx + (int)threadIdx.x % 3 - 1, y = ty + (int)threadIdx.x / 3 - 1;
-    if (x >= 0 && x < tiles_x && y >= 0 && y < tiles_y) wet = a.tile_wet_step[par * nt + y * tiles_x + x] != 0;
+__device__ __forceinline__ unsigned mask_tiles_to_do(const KArgs<R>& a, int t0, int ng, int tiles_x, int tiles_y) {
+  __shared__ uint8_t s_do[8];
+  const int nt = tiles_x * tiles_y;
+  RunState* st = a.st;
+  const unsigned par = (unsigned)(st->steps & 1);
+  if (threadIdx.x < (unsigned)((ng + 1) / 2 * 32)) {   // whole warps
+    const int g = threadIdx.x / 16, nb = threadIdx.x % 16, t = t0 + g;
+    int wet = 0;
+    uint8_t ta = 0, ts = 0;
+    if (g < ng) {
+      const int x = t % tiles_x + nb % 3 - 1, y = t / tiles_x + nb / 3 - 1;
+      if (nb < 9 && x >= 0 && x < tiles_x && y >= 0 && y < tiles_y) wet = a.tile_wet_step[par * nt + y * tiles_x + x] != 0;
+      if (nb == 0) {
+        ta = a.tile_active[t];
+        ts = a.tile_static[t];
+      }
+    }
+    const unsigned any_wet = (__ballot_sync(0xffffffffu, wet) >> (threadIdx.x & 16u)) & 0xffffu;
+    if (g < ng && nb == 0) {
+      a.tile_wet_step[(par ^ 1u) * nt + t] = 0;
+      const bool todo = any_wet || !(ta == TILE_DRY_BORDER || (ta == 0 && !(ts & TILE_SEED)));
+      s_do[g] = (uint8_t)((todo ? 1 : 0) | (ts & TILE_SPECIAL));
+      if (!todo && ta == TILE_DRY_BORDER) {
+        atomicAdd((unsigned long long*)&st->cells_acc[par], (unsigned long long)a.tile_count[t]);
+        atomicAdd(&st->border_acc[par], (unsigned long long)a.tile_count[t]);
+      }
+    }
   }
-  const uint8_t ta = a.tile_active[t];
-  const bool any_wet = __syncthreads_or(wet) != 0;
-  if (threadIdx.x == 0) a.tile_wet_step[(par ^ 1u) * nt + t] = 0;
-  const bool skip = (ta == TILE_DRY_BORDER || (ta == 0 && !a.tile_static[t])) && !any_wet;
-  if (skip && ta == TILE_DRY_BORDER && threadIdx.x == 0) {
-    atomicAdd((unsigned long long*)&a.st->cells_acc[a.st->steps & 1], (unsigned long long)a.tile_count[t]);
-    atomicAdd(&a.st->border_acc[a.st->steps & 1], (unsigned long long)a.tile_count[t]);
-  }
-  return skip;
+  __syncthreads();
+  unsigned todo = 0u;
+  for (int g = 0; g < ng; ++g) todo |= (unsigned)(s_do[g] & 1) << g | (unsigned)(s_do[g] >> 1) << (8 + g);
+  return todo;
+}
+
+// Tiles per block of k_mask for `tiles` tiles: one while every tile's block
+// can be resident (eight blocks of 256 threads per SM), then up to eight, so
+// that the many tiles that are skipped cost a sixteenth of a warp each instead
+// of a block, whose launch and first loads took most of the kernel on a large
+// domain.
+static inline int mask_group(int64_t tiles, int sms) {
+  int g = 1;
+  while (g < 8 && tiles > (int64_t)8 * sms * g) g *= 2;
+  return g;
 }
 
 // Time factor and inflow velocity of the bottom radial source at `time`
@@ -434,17 +513,35 @@ __device__ __forceinline__ void source_factors(const KArgs<R>& a, RunState* st, 
 }
 
 // mode 0: check_solve(.FALSE.); 1: check_solve(.TRUE.) (solve_all); 2: as 0
-// with the tile skip of mask_tile_skippable (the N_RK = 2 step, whose stage
+// with the tile skip of mask_tiles_to_do (the N_RK = 2 step, whose stage
 // kernel keeps the wet flags)
+// group: tiles per block, consecutive in the row-major order of the tiles
+// (mask_group).  Bound by instructions on the tiles it evaluates, by latency on
+// the ones it skips.  Measured with one tile per block and mask_tile for every
+// tile -> now: 4096^2 current (65,536 tiles, 8 a block) 135 -> 57 us, 1024^2
+// (4,096, 4 a block) 19.9 -> 15.1 (mask_tile in groups: 70 and 19.9).
 template <class R, int TH>
-__global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask(KArgs<R> a, int mode) {
+__global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask(KArgs<R> a, int mode, int tiles_x, int tiles_y,
+                                                                      int group) {
   step_kernel_entry();
   RunState* st = a.st;
   const double t = st->t;
   if (!running(st)) return;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) source_factors(a, st, t);
-  if (mode == 2 && mask_tile_skippable(a, blockIdx.x, blockIdx.y, gridDim.x, gridDim.y)) return;
-  mask_tile<R, TH>(a, mode == 1, blockIdx.x, blockIdx.y, gridDim.x, mode == 2);
+  const int t0 = blockIdx.x * group, ng = min(group, tiles_x * tiles_y - t0);
+  if (ng <= 0) {
+    // the block after the last (runs with a source only): the FP64 chain of
+    // the source factors, beside the tiles instead of before them
+    if (threadIdx.x == 0) source_factors(a, st, t);
+    return;
+  }
+  unsigned todo = 0xff00u | ((1u << ng) - 1u);
+  if (mode == 2) todo = mask_tiles_to_do(a, t0, ng, tiles_x, tiles_y);
+  for (unsigned m = todo & 0xffu; m; m &= m - 1u) {
+    const int g = __ffs(m) - 1, tile = t0 + g, tx = tile % tiles_x, ty = tile / tiles_x;
+    if (!((todo >> (8 + g)) & 1u)) mask_tile_plain<R, TH>(a, tx, ty, tiles_x, nullptr);
+    else mask_tile<R, TH>(a, mode == 1, tx, ty, tiles_x, mode == 2);
+    __syncthreads();   // shared memory of mask_tile is free
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1132,30 +1229,50 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
 // ---------------------------------------------------------------------------
 // k_dt: dt of this step (timestep + IMEX_SfloW2D.f90:417-439), one thread.
 // ---------------------------------------------------------------------------
+// The kernel is one chain of latencies, so every value is loaded before any
+// is used, and the accumulators that the blocks of the kernels before added to
+// with atomics are read (from L2) and cleared by plain accesses: no other
+// kernel touches them meanwhile.
 __device__ __forceinline__ void dt_update(RunState* st, double max_dt) {
-  if (!running(st)) { st->run_step = 0; return; }
-  // the CFL minimum and the active count were accumulated with atomics by
-  // the blocks of the kernels before: read and reset them with atomics
-  double dtmin = __longlong_as_double((long long)atomicExch(&st->dtmin_bits, dbits(1.0e300)));
+  const double t = st->t, dt_old = st->dt_old, dt_old_old = st->dt_old_old, t_end = st->t_end, t_stop = st->t_stop;
+  double t_output = st->t_output;
+  const long long steps = st->steps, step_limit = st->step_limit;
+  const long long cells_total = st->cells_total, border_total = st->border_total;
+  const unsigned long long min_bits = __ldcg(&st->dtmin_bits);
+  const unsigned long long c0 = __ldcg(&st->cells_acc[0]), c1 = __ldcg(&st->cells_acc[1]);
+  const unsigned long long b0 = __ldcg(&st->border_acc[0]), b1 = __ldcg(&st->border_acc[1]);
+  const unsigned status = st->status;
+  // running(st)
+  if (!(order_key(t) < order_key(t_stop) && steps < step_limit && !(status & SFLOW_S_FATAL))) {
+    st->run_step = 0;
+    return;
+  }
+  const double dtmin = __longlong_as_double((long long)min_bits);
   double dt = max_dt;
   if (dtmin < dt) dt = dtmin;
-  if (st->t_end - st->t_output < 1.0e-7) st->t_output = st->t_end;
-  if (st->t + dt > st->t_end) dt = st->t_end - st->t;
-  if (st->t + dt > st->t_output) dt = st->t_output - st->t;
-  double lim = 1.1 * 0.5 * (st->dt_old + st->dt_old_old);
+  if (t_end - t_output < 1.0e-7) {
+    t_output = t_end;
+    st->t_output = t_output;
+  }
+  if (t + dt > t_end) dt = t_end - t;
+  if (t + dt > t_output) dt = t_output - t;
+  const double lim = 1.1 * 0.5 * (dt_old + dt_old_old);
   if (lim < dt) dt = lim;
-  st->dt_old_old = st->dt_old;
+  st->dtmin_bits = dbits(1.0e300);
+  st->dt_old_old = dt_old;
   st->dt_old = dt;
   st->dt = dt;
-  st->t_prev = st->t;
-  st->t = st->t + dt;
+  st->t_prev = t;
+  st->t = t + dt;
   st->run_step = 1;
-  const int p = (int)(st->steps & 1);
-  const unsigned long long cells = atomicExch(&st->cells_acc[p], 0ull);
+  const int p = (int)(steps & 1);
+  const unsigned long long cells = p ? c1 : c0;
   st->last_cells = (long long)cells;
-  st->cells_total += (long long)cells;
-  st->border_total += (long long)atomicExch(&st->border_acc[p], 0ull);
-  st->steps += 1;
+  st->cells_total = cells_total + (long long)cells;
+  st->border_total = border_total + (long long)(p ? b1 : b0);
+  st->cells_acc[p] = 0ull;
+  st->border_acc[p] = 0ull;
+  st->steps = steps + 1;
 }
 
 static __global__ void k_dt(RunState* st, double max_dt) {

@@ -1113,23 +1113,33 @@ class Solver : public SolverBase {
     }
     return e;
   }
-  // tiles with a border cell, a ring-boundary cell or a bottom-source cell
-  // (seeds of every check_solve) within n_RK cells
+  // TILE_SEED: a border, ring-boundary or bottom-source cell (seeds of every
+  // check_solve) within n_RK cells; TILE_SPECIAL: one, or a ring-interior
+  // cell, within the 4-cell frame of check_solve
   std::vector<uint8_t> tile_static_host() const {
-    const int nx = hs_.nx, ny = hs_.ny, r = hs_.nrk, th = tile_h_;
+    const int nx = hs_.nx, ny = hs_.ny, th = tile_h_;
     std::vector<uint8_t> ts((size_t)tiles_x_ * tiles_y_, 0);
     for (int ty = 0; ty < tiles_y_; ++ty)
       for (int tx = 0; tx < tiles_x_; ++tx) {
-        const int j0 = tx * TX - r, j1 = std::min(nx, (tx + 1) * TX) - 1 + r;
-        const int k0 = ty * th - r, k1 = std::min(ny, (ty + 1) * th) - 1 + r;
-        uint8_t v = (j0 <= 0 || j1 >= nx - 1 || k0 <= 0 || k1 >= ny - 1) ? 1 : 0;
-        if (!v && (hs_.p.radial_source_flag || hs_.p.bottom_radial_source_flag))
-          for (int k = std::max(k0, 0); k <= std::min(k1, ny - 1) && !v; ++k)
-            for (int j = std::max(j0, 0); j <= std::min(j1, nx - 1); ++j) {
-              const uint8_t f = hs_.cflags[(size_t)k * nx + j];
-              if ((f & 3) == 2 || (f & kFlagBottom)) { v = 1; break; }
-            }
-        ts[(size_t)ty * tiles_x_ + tx] = v;
+        auto near_border = [&](int r) {
+          return tx * TX - r <= 0 || std::min(nx, (tx + 1) * TX) - 1 + r >= nx - 1 || ty * th - r <= 0 ||
+                 std::min(ny, (ty + 1) * th) - 1 + r >= ny - 1;
+        };
+        ts[(size_t)ty * tiles_x_ + tx] =
+            (uint8_t)((near_border(hs_.nrk) ? TILE_SEED : 0) | (near_border(MASK_HALO) ? TILE_SPECIAL : 0));
+      }
+    if (!hs_.p.radial_source_flag && !hs_.p.bottom_radial_source_flag) return ts;
+    auto mark = [&](int j, int k, int r, uint8_t bit) {
+      for (int ty = std::max(k - r, 0) / th; ty <= std::min(k + r, ny - 1) / th; ++ty)
+        for (int tx = std::max(j - r, 0) / TX; tx <= std::min(j + r, nx - 1) / TX; ++tx)
+          ts[(size_t)ty * tiles_x_ + tx] |= bit;
+    };
+    for (int k = 0; k < ny; ++k)
+      for (int j = 0; j < nx; ++j) {
+        const uint8_t f = hs_.cflags[(size_t)k * nx + j];
+        if (!((f & 3) || (f & kFlagBottom))) continue;
+        mark(j, k, MASK_HALO, TILE_SPECIAL);
+        if ((f & 3) == 2 || (f & kFlagBottom)) mark(j, k, hs_.nrk, TILE_SEED);
       }
     return ts;
   }

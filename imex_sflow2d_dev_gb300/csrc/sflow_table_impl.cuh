@@ -135,7 +135,14 @@ static inline dim3 stage_grid(dim3 tiles, int ny) {
 
 template <class R, int NS, int TH>
 static cudaError_t tab_mask(const KArgs<R>& a, dim3 grid, cudaStream_t s, int solve_all) {
-  return launch_step_kernel(k_mask<R, TH>, grid, dim3(TileShape<TH>::MASK_THREADS), 0, s, a.g.pdl, a, solve_all);
+  int sms = 0;
+  const cudaError_t e = sm_count(&sms);
+  if (e != cudaSuccess) return e;
+  const int64_t tiles = (int64_t)grid.x * grid.y;
+  const int group = mask_group(tiles, sms);
+  return launch_step_kernel(k_mask<R, TH>, dim3((unsigned)((tiles + group - 1) / group) + (a.pd.radial_source || a.pd.bottom_source ? 1u : 0u)),
+                            dim3(TileShape<TH>::MASK_THREADS), 0, s, a.g.pdl, a, solve_all, (int)grid.x, (int)grid.y,
+                            group);
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStream_t s, const R* qin,
