@@ -73,6 +73,15 @@ __device__ __forceinline__ void recon64(const double* v, int sv, const double* q
   }
 }
 
+// the other cells (domain edge, ring inlet), and every cell of other limiters
+// (out of line, through memory: here the state is better off in local memory
+// than in the registers of the FP64 arithmetic)
+template <int NS, int DIR, int LIM>
+__device__ __noinline__ void recon64_other(const KArgs<double>& a, const double* sqp, const uint8_t* sfl, int rx,
+                                           int ry, int j, int k, int plus, double* out) {
+  recon_side<double, NS, DIR, LIM, 8>(a, sqp, sfl, rx, ry, j, k, plus, out);
+}
+
 // face_flux with recon64 for the ordinary cells: qf points at the divided
 // differences of this face, step to those of the next face along DIR
 template <int NS, int DIR, int LIM>
@@ -99,14 +108,14 @@ __device__ __forceinline__ double face_flux64(const KArgs<double>& a, const doub
     if (LIM == 1 && f - 1 > 0 && f < n && !src_l)
       recon64<NS>(sqp + ryl * RX + rxl, kFlux64Plane, qf - step, qf, sq, kd, 1, qpl);
     else
-      recon_side<double, NS, DIR, LIM, 8>(a, sqp, sfl, rxl, ryl, (DIR == 1) ? f - 1 : o, (DIR == 1) ? o : f - 1, 1, qpl);
+      recon64_other<NS, DIR, LIM>(a, sqp, sfl, rxl, ryl, (DIR == 1) ? f - 1 : o, (DIR == 1) ? o : f - 1, 1, qpl);
     hl = true;
   }
   if (f < n && acth && !mirror_h) {
     if (LIM == 1 && f > 0 && f < n - 1 && !src_h)
       recon64<NS>(sqp + ryh * RX + rxh, kFlux64Plane, qf, qf + step, sq, kd, 0, qph);
     else
-      recon_side<double, NS, DIR, LIM, 8>(a, sqp, sfl, rxh, ryh, (DIR == 1) ? f : o, (DIR == 1) ? o : f, 0, qph);
+      recon64_other<NS, DIR, LIM>(a, sqp, sfl, rxh, ryh, (DIR == 1) ? f : o, (DIR == 1) ? o : f, 0, qph);
     hh = true;
   }
   if (f == 0) {

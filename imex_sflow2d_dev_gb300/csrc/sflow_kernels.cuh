@@ -459,13 +459,34 @@ __device__ __forceinline__ unsigned mask_tiles_to_do(const KArgs<R>& a, int t0, 
 
 // Tiles per block of k_mask for `tiles` tiles: one while every tile's block
 // can be resident (eight blocks of 256 threads per SM), then up to eight, so
-// that the many tiles that are skipped cost a sixteenth of a warp each instead
-// of a block, whose launch and first loads took most of the kernel on a large
+// that the many tiles that are skipped cost half a warp each instead of a
+// block, whose launch and first loads took most of the kernel on a large
 // domain.
 static inline int mask_group(int64_t tiles, int sms) {
   int g = 1;
   while (g < 8 && tiles > (int64_t)8 * sms * g) g *= 2;
   return g;
+}
+
+// The skip test of one tile for a whole block (block-uniform).
+template <class R>
+__device__ __forceinline__ bool mask_tile_skippable(const KArgs<R>& a, int tx, int ty, int tiles_x, int tiles_y) {
+  const int nt = tiles_x * tiles_y, t = ty * tiles_x + tx;
+  const unsigned par = (unsigned)(a.st->steps & 1);
+  int wet = 0;
+  if (threadIdx.x < 9) {
+    const int x = tx + (int)threadIdx.x % 3 - 1, y = ty + (int)threadIdx.x / 3 - 1;
+    if (x >= 0 && x < tiles_x && y >= 0 && y < tiles_y) wet = a.tile_wet_step[par * nt + y * tiles_x + x] != 0;
+  }
+  const uint8_t ta = a.tile_active[t];
+  const bool any_wet = __syncthreads_or(wet) != 0;
+  if (threadIdx.x == 0) a.tile_wet_step[(par ^ 1u) * nt + t] = 0;
+  const bool skip = (ta == TILE_DRY_BORDER || (ta == 0 && !(a.tile_static[t] & TILE_SEED))) && !any_wet;
+  if (skip && ta == TILE_DRY_BORDER && threadIdx.x == 0) {
+    atomicAdd((unsigned long long*)&a.st->cells_acc[a.st->steps & 1], (unsigned long long)a.tile_count[t]);
+    atomicAdd(&a.st->border_acc[a.st->steps & 1], (unsigned long long)a.tile_count[t]);
+  }
+  return skip;
 }
 
 // Time factor and inflow velocity of the bottom radial source at `time`
@@ -513,34 +534,49 @@ __device__ __forceinline__ void source_factors(const KArgs<R>& a, RunState* st, 
 }
 
 // mode 0: check_solve(.FALSE.); 1: check_solve(.TRUE.) (solve_all); 2: as 0
-// with the tile skip of mask_tiles_to_do (the N_RK = 2 step, whose stage
+// with the tile skip of mask_tile_skippable (the N_RK = 2 step, whose stage
 // kernel keeps the wet flags)
-// group: tiles per block, consecutive in the row-major order of the tiles
-// (mask_group).  Bound by instructions on the tiles it evaluates, by latency on
-// the ones it skips.  Measured with one tile per block and mask_tile for every
-// tile -> now: 4096^2 current (65,536 tiles, 8 a block) 135 -> 57 us, 1024^2
-// (4,096, 4 a block) 19.9 -> 15.1 (mask_tile in groups: 70 and 19.9).
+// A run with a source launches one block more (row tiles_y): it evaluates the
+// FP64 chain of the source factors beside the tiles instead of before them.
 template <class R, int TH>
-__global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask(KArgs<R> a, int mode, int tiles_x, int tiles_y,
-                                                                      int group) {
+__global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask(KArgs<R> a, int mode, int tiles_y) {
+  step_kernel_entry();
+  RunState* st = a.st;
+  const double t = st->t;
+  if (!running(st)) return;
+  if ((int)blockIdx.y == tiles_y) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) source_factors(a, st, t);
+    return;
+  }
+  if (mode == 2 && mask_tile_skippable(a, blockIdx.x, blockIdx.y, gridDim.x, tiles_y)) return;
+  mask_tile<R, TH>(a, mode == 1, blockIdx.x, blockIdx.y, gridDim.x, mode == 2);
+}
+
+// check_solve of the N_RK = 2 step (mode 2) on a large domain: `group` tiles
+// per block, consecutive in the row-major order of the tiles (mask_group).
+// Bound by instructions on the tiles it evaluates, by latency on the ones it
+// skips.  Measured with k_mask -> this kernel: 4096^2 current (65,536 tiles, 8
+// a block) 135 -> 57 us, 1024^2 (4,096, 4 a block) 19.9 -> 15.1 (without
+// mask_tile_plain 70 and 19.9).  On a small domain, one tile a block, its
+// longer code made it 1 us slower (64^2 9.5 -> 10.5 us), so those keep k_mask.
+template <class R, int TH>
+__global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask_group(KArgs<R> a, int tiles_x, int tiles_y,
+                                                                            int group) {
   step_kernel_entry();
   RunState* st = a.st;
   const double t = st->t;
   if (!running(st)) return;
   const int t0 = blockIdx.x * group, ng = min(group, tiles_x * tiles_y - t0);
-  if (ng <= 0) {
-    // the block after the last (runs with a source only): the FP64 chain of
-    // the source factors, beside the tiles instead of before them
+  if (ng <= 0) {   // the block after the last (see k_mask)
     if (threadIdx.x == 0) source_factors(a, st, t);
     return;
   }
-  unsigned todo = 0xff00u | ((1u << ng) - 1u);
-  if (mode == 2) todo = mask_tiles_to_do(a, t0, ng, tiles_x, tiles_y);
+  const unsigned todo = mask_tiles_to_do(a, t0, ng, tiles_x, tiles_y);
   for (unsigned m = todo & 0xffu; m; m &= m - 1u) {
     const int g = __ffs(m) - 1, tile = t0 + g, tx = tile % tiles_x, ty = tile / tiles_x;
     if (!((todo >> (8 + g)) & 1u)) mask_tile_plain<R, TH>(a, tx, ty, tiles_x, nullptr);
-    else mask_tile<R, TH>(a, mode == 1, tx, ty, tiles_x, mode == 2);
-    __syncthreads();   // shared memory of mask_tile is free
+    else mask_tile<R, TH>(a, 0, tx, ty, tiles_x, true);
+    __syncthreads();   // shared memory of the tile's masks is free
   }
 }
 
@@ -615,9 +651,15 @@ __device__ __forceinline__ R slope(R v0, R v1, R v2, const Spacing<R>& s, int li
 // reference's use of y_stag in the x slope of v at ring cells with a ring
 // face to the north only (solver_2d.f90:3605, kept as is).
 // ---------------------------------------------------------------------------
+// (Returned by value: a pointer to the caller's array would keep every face's
+// state in local memory.)
+template <class R, int NS>
+struct QpSide {
+  R v[4 + NS + 2];
+};
 template <class R, int NS, int DIR, int LIM, int TH>
-__device__ __noinline__ void recon_side_edge(const KArgs<R>& a, const R* sqp, const uint8_t* sfl,
-                                           int rx, int ry, int j, int k, int plus, R* out) {
+__device__ __noinline__ QpSide<R, NS> recon_side_edge(const KArgs<R>& a, const R* sqp, const uint8_t* sfl,
+                                                      int rx, int ry, int j, int k, int plus) {
   constexpr int nv = 4 + NS, np = nv + 2;
   const Grid<R>& g = a.g;
   constexpr int plane = RX * TileShape<TH>::RY;
@@ -732,8 +774,10 @@ __device__ __noinline__ void recon_side_edge(const KArgs<R>& a, const R* sqp, co
 #pragma unroll
     for (int i = 0; i < np; ++i) qm[i] = cell[i];
   }
+  QpSide<R, NS> out;
 #pragma unroll
-  for (int i = 0; i < np; ++i) out[i] = qm[i];
+  for (int i = 0; i < np; ++i) out.v[i] = qm[i];
+  return out;
 }
 
 // Interior cells without a ring face (almost every cell): three-point
@@ -742,19 +786,10 @@ __device__ __noinline__ void recon_side_edge(const KArgs<R>& a, const R* sqp, co
 // the edge version is a separate (not inlined) function so that the face
 // code every thread runs stays small.
 template <class R, int NS, int DIR, int LIM, int TH>
-__device__ __forceinline__ void recon_side(const KArgs<R>& a, const R* sqp, const uint8_t* sfl,
-                                           int rx, int ry, int j, int k, int plus, R* out) {
-  constexpr int nv = 4 + NS, np = nv + 2;
+__device__ __forceinline__ void recon_ordinary(const KArgs<R>& a, const R* sqp, int rx, int ry, int c, int plus, R* out) {
+  constexpr int np = 4 + NS + 2;
   const Grid<R>& g = a.g;
   constexpr int plane = RX * TileShape<TH>::RY;
-  const int n = (DIR == 1) ? g.nx : g.ny;
-  const int c = (DIR == 1) ? j : k;
-  const uint8_t fl = sfl[ry * RX + rx];
-  const bool src2 = a.pr.radial_source && (fl & F_SC_MASK) == 2;
-  if (c == 0 || c == n - 1 || src2) {
-    recon_side_edge<R, NS, DIR, LIM, TH>(a, sqp, sfl, rx, ry, j, k, plus, out);
-    return;
-  }
   auto QP = [&](int i, int o) -> R {
     return (DIR == 1) ? sqp[i * plane + ry * RX + (rx + o)] : sqp[i * plane + (ry + o) * RX + rx];
   };
@@ -781,6 +816,22 @@ __device__ __forceinline__ void recon_side(const KArgs<R>& a, const R* sqp, cons
     const R dq = g.rc * d2 * sl;
     out[i] = plus ? v1 + dq : v1 - dq;
   }
+}
+
+template <class R, int NS, int DIR, int LIM, int TH>
+__device__ __forceinline__ void recon_side(const KArgs<R>& a, const R* sqp, const uint8_t* sfl,
+                                           int rx, int ry, int j, int k, int plus, R* out) {
+  const int n = (DIR == 1) ? a.g.nx : a.g.ny;
+  const int c = (DIR == 1) ? j : k;
+  const uint8_t fl = sfl[ry * RX + rx];
+  const bool src2 = a.pr.radial_source && (fl & F_SC_MASK) == 2;
+  if (c == 0 || c == n - 1 || src2) {
+    const QpSide<R, NS> r = recon_side_edge<R, NS, DIR, LIM, TH>(a, sqp, sfl, rx, ry, j, k, plus);
+#pragma unroll
+    for (int i = 0; i < 4 + NS + 2; ++i) out[i] = r.v[i];
+    return;
+  }
+  recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rx, ry, c, plus, out);
 }
 
 // One side of a face reduced to what the KT flux needs.
@@ -910,13 +961,18 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
   return rmax(a2, -a1);
 }
 
-// One face along DIR between the low cell (f-1) and the high cell (f):
-// reconstruction of both sides, the domain-edge copies and the wall mirror
-// at ring-inlet faces (solver_2d.f90:3716-3920), KT flux.  Returns the
-// largest |speed| at the face (a_interface_*_max).
+// Both sides of a face of a special tile (domain edge, ring inlet or source
+// nearby): reconstruction, the domain-edge copies and the wall mirror at
+// ring-inlet faces (solver_2d.f90:3716-3920).  flags: bit 0 / 1 the low / high
+// side exists, bit 2 / 3 it is a wall mirror.
+template <class R, int NS>
+struct FaceStates {
+  R lo[4 + NS + 2], hi[4 + NS + 2];
+  int flags;
+};
 template <class R, int NS, int DIR, int LIM, int TH>
-__device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f,
-                                       int o, int rxl, int ryl, int rxh, int ryh, R gcs, R* H) {
+__device__ __noinline__ FaceStates<R, NS> face_states_special(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f,
+                                                              int o, int rxl, int ryl, int rxh, int ryh) {
   constexpr int nv = 4 + NS, np = nv + 2;
   constexpr int vel = (DIR == 1) ? nv : nv + 1;
   const int n = (DIR == 1) ? a.g.nx : a.g.ny;
@@ -928,7 +984,9 @@ __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const ui
   const bool ring_h = radial && (flh & F_SC_MASK) == 2 && f > 0 && f < n - 1;
   const bool mirror_h = actl && ring_l && ((DIR == 1) ? (fll & F_E) : ((fll & F_N) && !(fll & F_S)));
   const bool mirror_l = !mirror_h && acth && ring_h && ((DIR == 1) ? ((flh & F_W) && !(flh & F_E)) : (flh & F_S));
-  R qpl[np], qph[np];
+  FaceStates<R, NS> s;
+  R* qpl = s.lo;
+  R* qph = s.hi;
   bool hl = false, hh = false;
   const int jl = (DIR == 1) ? f - 1 : o, kl = (DIR == 1) ? o : f - 1;
   const int jh = (DIR == 1) ? f : o, kh = (DIR == 1) ? o : f;
@@ -956,10 +1014,45 @@ __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const ui
     qpl[vel] = -qpl[vel];
     hl = true;
   }
+  s.flags = (hl ? 1 : 0) | (hh ? 2 : 0) | (mirror_l ? 4 : 0) | (mirror_h ? 8 : 0);
+  return s;
+}
+
+// One face along DIR between the low cell (f-1) and the high cell (f):
+// reconstruction of both sides, KT flux.  Returns the largest |speed| at the
+// face (a_interface_*_max).  plain (block-uniform): no domain edge, ring or
+// source cell in the tile's region, so both cells are ordinary.  (An inactive
+// cell holds no mass, and no neighbour of it does: its reconstructed state is
+// the dry one that an absent side has.)
+// The kernel is bound by instructions, two thirds of them not arithmetic; the
+// special faces' rules and their states in local memory were part of it for
+// every face.  With them out of line and passed by value, and 4 blocks per SM
+// (56 registers, a few spills; the generic-limiter kernel is faster with its
+// 72 registers and 3 blocks): k_flux 47.4 -> 43.1 us on a 1024^2 current, 328
+// -> 284 on a 4096^2 one, k_b_flux 58 -> 50 on an ensemble of 64 floods; the
+// same bits.
+template <class R, int NS, int DIR, int LIM, int TH>
+__device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, bool plain, int f,
+                                       int o, int rxl, int ryl, int rxh, int ryh, R gcs, R* H) {
+  constexpr int np = 4 + NS + 2;
+  R qpl[np], qph[np];
+  int flags = 3;
+  if (plain) {
+    recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxl, ryl, f - 1, 1, qpl);
+    recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxh, ryh, f, 0, qph);
+  } else {
+    const FaceStates<R, NS> s = face_states_special<R, NS, DIR, LIM, TH>(a, sqp, sfl, f, o, rxl, ryl, rxh, ryh);
+#pragma unroll
+    for (int i = 0; i < np; ++i) {
+      qpl[i] = s.lo[i];
+      qph[i] = s.hi[i];
+    }
+    flags = s.flags;
+  }
   Side<R, NS> L, Hs;
-  if (hl) side_from_qp<R, NS, DIR>(a, qpl, gcs, L, mirror_l);
+  if (flags & 1) side_from_qp<R, NS, DIR>(a, qpl, gcs, L, flags & 4);
   else side_zero(L);
-  if (hh) side_from_qp<R, NS, DIR>(a, qph, gcs, Hs, mirror_h);
+  if (flags & 2) side_from_qp<R, NS, DIR>(a, qph, gcs, Hs, flags & 8);
   else side_zero(Hs);
   if (a.pr.scheme == SFLOW_SCHEME_UP) return up_flux<R, NS, DIR>(L, Hs, H);
   return kt_flux<R, NS, DIR>(L, Hs, H);
@@ -991,6 +1084,7 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
   uint8_t* sfl = reinterpret_cast<uint8_t*>(sgeo + 5 * TX * TY);  // RX*RY
   const int j0 = tx * TX, k0 = ty * TY;
   const int tid = threadIdx.x;
+  const bool plain = !(a.tile_static[ty * g.tiles_x + tx] & TILE_SPECIAL);
 
   __syncthreads();   // shared memory of the previous tile of a persistent block is free
   // 0. the topography terms of the cell this thread finishes in step 4
@@ -1099,10 +1193,10 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
     if (any) {
       const int64_t cl = cidx(g, f > 0 ? f - 1 : 0, k), ch = cidx(g, f < g.nx ? f : g.nx - 1, k);
       R gcs;
-      if (f == 0) gcs = __ldg(a.geo[5] + ch);
-      else if (f == g.nx) gcs = __ldg(a.geo[5] + cl);
+      if (!plain && f == 0) gcs = __ldg(a.geo[5] + ch);
+      else if (!plain && f == g.nx) gcs = __ldg(a.geo[5] + cl);
       else gcs = cst<R>(0.5) * (__ldg(a.geo[5] + cl) + __ldg(a.geo[5] + ch));
-      amax = face_flux<R, NS, 1, LIM, TH>(a, sqp, sfl, f, k, rxl, ry, rxh, ry, gcs, H);
+      amax = face_flux<R, NS, 1, LIM, TH>(a, sqp, sfl, plain, f, k, rxl, ry, rxh, ry, gcs, H);
     } else {
 #pragma unroll
       for (int i = 0; i < nv; ++i) H[i] = R(0);
@@ -1130,10 +1224,10 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
     if (any) {
       const int64_t cl = cidx(g, j, f > 0 ? f - 1 : 0), ch = cidx(g, j, f < g.ny ? f : g.ny - 1);
       R gcs;
-      if (f == 0) gcs = __ldg(a.geo[5] + ch);
-      else if (f == g.ny) gcs = __ldg(a.geo[5] + cl);
+      if (!plain && f == 0) gcs = __ldg(a.geo[5] + ch);
+      else if (!plain && f == g.ny) gcs = __ldg(a.geo[5] + cl);
       else gcs = cst<R>(0.5) * (__ldg(a.geo[5] + cl) + __ldg(a.geo[5] + ch));
-      amax = face_flux<R, NS, 2, LIM, TH>(a, sqp, sfl, f, j, rx, ryl, rx, ryh, gcs, H);
+      amax = face_flux<R, NS, 2, LIM, TH>(a, sqp, sfl, plain, f, j, rx, ryl, rx, ryh, gcs, H);
     } else {
 #pragma unroll
       for (int i = 0; i < nv; ++i) H[i] = R(0);
@@ -1281,8 +1375,8 @@ static __global__ void k_dt(RunState* st, double max_dt) {
 }
 
 template <class R, int NS, int LIM, int TH>
-__global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS) k_flux(KArgs<R> a, const R* __restrict__ qin,
-                                                       R* __restrict__ rout, int want_dt) {
+__global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, LIM == 1 ? TileShape<TH>::FLUX_MIN_BLOCKS : 1)
+    k_flux(KArgs<R> a, const R* __restrict__ qin, R* __restrict__ rout, int want_dt) {
   step_kernel_entry();
   const RunState* st = a.st;
   extern __shared__ __align__(16) unsigned char smem_raw[];

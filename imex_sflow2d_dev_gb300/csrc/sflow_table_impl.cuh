@@ -135,14 +135,18 @@ static inline dim3 stage_grid(dim3 tiles, int ny) {
 
 template <class R, int NS, int TH>
 static cudaError_t tab_mask(const KArgs<R>& a, dim3 grid, cudaStream_t s, int solve_all) {
+  const dim3 T(TileShape<TH>::MASK_THREADS);
+  const int tx = (int)grid.x, ty = (int)grid.y;
+  const unsigned src = a.pd.radial_source || a.pd.bottom_source ? 1u : 0u;
+  const int64_t tiles = (int64_t)tx * ty;
   int sms = 0;
   const cudaError_t e = sm_count(&sms);
   if (e != cudaSuccess) return e;
-  const int64_t tiles = (int64_t)grid.x * grid.y;
   const int group = mask_group(tiles, sms);
-  return launch_step_kernel(k_mask<R, TH>, dim3((unsigned)((tiles + group - 1) / group) + (a.pd.radial_source || a.pd.bottom_source ? 1u : 0u)),
-                            dim3(TileShape<TH>::MASK_THREADS), 0, s, a.g.pdl, a, solve_all, (int)grid.x, (int)grid.y,
-                            group);
+  if (group == 1 || solve_all != 2)
+    return launch_step_kernel(k_mask<R, TH>, dim3(grid.x, grid.y + src), T, 0, s, a.g.pdl, a, solve_all, ty);
+  return launch_step_kernel(k_mask_group<R, TH>, dim3((unsigned)((tiles + group - 1) / group) + src), T, 0, s, a.g.pdl,
+                            a, tx, ty, group);
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStream_t s, const R* qin,
