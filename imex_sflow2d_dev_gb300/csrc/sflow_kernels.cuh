@@ -46,9 +46,15 @@ struct TileShape {
 constexpr int kTileHDefault = 8;
 
 // Thread blocks of a single run's pointwise kernels: 32 x ROWS cells, one
-// cell each, of one tile (or half a tile of 32 x 4).
-//  FP32: 8 rows, 6 blocks per SM (40 registers): the stage waits on memory,
-//        and more warps hide more of it.
+// cell each, of one tile (or half a tile of 32 x 4).  k_stage2:
+//  FP32, SMALL (the blocks of 8 rows number at most 8 per SM): 4 rows, 12
+//        blocks per SM (40 registers); the kernel is one wave that waits on
+//        memory, and smaller blocks spread the wet ones over the SMs (640 x
+//        480 current with settling 25.0 -> 22.5 us against 8 rows, 6 blocks).
+//  FP32, else: 8 rows, 4 blocks per SM (64 registers, no spills): 4096^2
+//        current with settling and entrainment 575 -> 526 us, 1024^2 30.6 ->
+//        30.0 against 6 blocks per SM (40 registers); 5 blocks 533 and 30.7, 3
+//        blocks 605 and 32.8.
 //  FP64: 2 rows, 4 blocks per SM (255 registers).  The stage is bound by
 //        FP64 instructions and the latency of their chains, both varying
 //        tenfold between warps (Newton and settling iterations, wet or dry),
@@ -60,7 +66,9 @@ template <class R>
 struct StageShape {
   static constexpr int ROWS = sizeof(R) == 4 ? 8 : 2;
   static constexpr int THREADS = TX * ROWS;
-  static constexpr int MIN_BLOCKS = sizeof(R) == 4 ? 6 : 4;
+  static constexpr int MIN_BLOCKS = 4;
+  static constexpr int SMALL_ROWS = sizeof(R) == 4 ? 4 : 2;
+  static constexpr int SMALL_MIN_BLOCKS = sizeof(R) == 4 ? 12 : 4;
 };
 
 // flag byte bits
@@ -2016,9 +2024,8 @@ constexpr uint8_t TW_ANY = 1, TW_W = 2, TW_E = 4, TW_S = 8, TW_N = 16;
 
 // single run: one block per 32 x ROWS cells (grid tiles_x x ceil(ny/ROWS));
 // the activity byte is the one of the 32 x TH tile holding the block.
-template <class R, int NS, int TH>
-__global__ void __launch_bounds__(StageShape<R>::THREADS, StageShape<R>::MIN_BLOCKS) k_stage2(KArgs<R> a, int mode) {
-  constexpr int ROWS = StageShape<R>::ROWS;
+template <class R, int NS, int TH, int ROWS, int MIN_BLOCKS>
+__global__ void __launch_bounds__(TX * ROWS, MIN_BLOCKS) k_stage2(KArgs<R> a, int mode) {
   step_kernel_entry();
   const bool go = a.st->run_step != 0;   // tested with the tile's code: one latency
   const int kk = blockIdx.y * ROWS + threadIdx.x / TX;

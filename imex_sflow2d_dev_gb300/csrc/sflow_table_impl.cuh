@@ -170,8 +170,18 @@ static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStrea
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_stage2(const KArgs<R>& a, dim3 grid, cudaStream_t s, int mode) {
-  return launch_step_kernel(k_stage2<R, NS, TH>, stage_grid<R>(grid, a.g.ny), dim3(StageShape<R>::THREADS), 0, s,
-                            a.g.pdl, a, mode);
+  using S = StageShape<R>;
+  if constexpr (S::SMALL_ROWS != S::ROWS) {
+    int sms = 0;
+    const cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    if ((int64_t)grid.x * ((a.g.ny + S::ROWS - 1) / S::ROWS) <= (int64_t)8 * sms)
+      return launch_step_kernel(k_stage2<R, NS, TH, S::SMALL_ROWS, S::SMALL_MIN_BLOCKS>,
+                                dim3(grid.x, (unsigned)((a.g.ny + S::SMALL_ROWS - 1) / S::SMALL_ROWS)),
+                                dim3(TX * S::SMALL_ROWS), 0, s, a.g.pdl, a, mode);
+  }
+  return launch_step_kernel(k_stage2<R, NS, TH, S::ROWS, S::MIN_BLOCKS>, stage_grid<R>(grid, a.g.ny), dim3(S::THREADS),
+                            0, s, a.g.pdl, a, mode);
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_stage(const KArgs<R>& a, dim3 grid, cudaStream_t s, int irk) {
