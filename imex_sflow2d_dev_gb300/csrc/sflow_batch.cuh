@@ -105,14 +105,13 @@ class Batch : public BatchBase {
     Solver<R>& sv = *pr->sv;
     sv.reserve_extra(sizeof(uint32_t) * (size_t)pr->tiles);
     sv.reserve_extra((size_t)pr->tiles);
-    *rc = sv.init();
-    if (*rc == SFLOW_OK) *rc = sv.upload(q_aos);
-    if (*rc == SFLOW_OK) *rc = sv.limits(pr->t_end, max_steps > 0 ? max_steps : -1);
+    *rc = sv.init(true);
+    if (*rc == SFLOW_OK) *rc = sv.upload(q_aos, true, pr->t_end, max_steps > 0 ? max_steps : -1);
     if (*rc != SFLOW_OK) {
       err = sv.err_;
+      cudaStreamSynchronize(sv.stream());   // nothing reads host arrays any more
       return nullptr;
     }
-    sv.trim_stage();
     const std::vector<uint8_t> ts = sv.tile_seed_host();
     pr->cand = static_cast<uint32_t*>(sv.carve(sizeof(uint32_t) * pr->tiles));
     pr->tile_seed = static_cast<uint8_t*>(sv.carve(ts.size()));
@@ -124,6 +123,7 @@ class Batch : public BatchBase {
       if (cudaMalloc((void**)&pr->cand, sizeof(uint32_t) * pr->tiles) != cudaSuccess ||
           cudaMalloc((void**)&pr->tile_seed, ts.size()) != cudaSuccess) {
         cudaGetLastError();
+        cudaStreamSynchronize(sv.stream());
         *rc = SFLOW_ENOMEM;
         err = "cudaMalloc failed";
         return nullptr;
@@ -131,11 +131,13 @@ class Batch : public BatchBase {
     }
     if (cudaMemsetAsync(pr->cand, 0, sizeof(uint32_t) * pr->tiles, sv.stream()) != cudaSuccess ||
         cudaMemcpyAsync(pr->tile_seed, ts.data(), ts.size(), cudaMemcpyHostToDevice, sv.stream()) != cudaSuccess ||
-        cudaStreamSynchronize(sv.stream()) != cudaSuccess) {
+        sv.finish_upload() != SFLOW_OK) {
+      cudaStreamSynchronize(sv.stream());
       *rc = SFLOW_ECUDA;
       err = "cudaMemcpy failed";
       return nullptr;
     }
+    sv.trim_stage();
     return pr;
   }
 
@@ -180,13 +182,12 @@ class Batch : public BatchBase {
       g->graph = nullptr;
     }
     // the batch stream is idle here (every advance ends synchronised)
-    if (cudaMemcpy(g->d_args + slot, &ka, sizeof(ka), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(g->d_runs + slot, &br, sizeof(br), cudaMemcpyHostToDevice) != cudaSuccess) {
-      err_ = "cudaMemcpy failed";
-      return SFLOW_ECUDA;
-    }
-    cudaError_t e = g->tab.b_admit(g->args, g->stream, slot, gen, (unsigned)tiles);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    // (one synchronisation for both copies and the list entry)
+    cudaError_t e = cudaMemcpyAsync(g->d_args + slot, &ka, sizeof(ka), cudaMemcpyHostToDevice, g->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_runs + slot, &br, sizeof(br), cudaMemcpyHostToDevice, g->stream);
+    if (e == cudaSuccess) e = g->tab.b_admit(g->args, g->stream, slot, gen, (unsigned)tiles);
+    const cudaError_t es = cudaStreamSynchronize(g->stream);   // the copies read this frame
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) { err_ = cudaGetErrorString(e); return SFLOW_ECUDA; }
     ++g->launches;
     s.gen = gen;
