@@ -702,8 +702,9 @@ __device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos,
   else return settling_velocity_inl<R>(P, diam, rhos, rhoc, inv_kin_visc);
 }
 
-// erodible: the cell's erodible solid thicknesses (null: none, as with
-// EROSION_COEFF = 0).  Returns the deposition and erosion rates (dep, ers),
+// settle: the classes' settling velocities where they are the run's constants
+// (k_settling), else null.  erodible: the cell's erodible solid thicknesses
+// (null: none, as with EROSION_COEFF = 0).  Returns the deposition and erosion rates (dep, ers),
 // the equation terms and the topography rate topo.  As in the reference the
 // erosion rates are set before the ALPHASTOT_MIN return, which leaves the
 // equation terms at zero.  With ERODIBLE_DEPOSIT_FLAG the erodible layer
@@ -711,7 +712,7 @@ __device__ __forceinline__ R settling_velocity(const Phys<R>& P, R diam, R rhos,
 // T_erodible to the cell's T just before this use).
 template <class R, int NS>
 __device__ __forceinline__ void mass_exchange(const Phys<R>& P, const R* qpj, R Bx, R By, R dt,
-                                              const R* erodible, R* dep, R* ers, R* eqn, R& topo,
+                                              const R* erodible, const R* settle, R* dep, R* ers, R* eqn, R& topo,
                                               unsigned* dep_limited = nullptr) {
   constexpr int ns = NS, nv = 4 + NS;
   for (int i = 0; i < ns; ++i) { dep[i] = R(0); ers[i] = R(0); }
@@ -740,13 +741,15 @@ __device__ __forceinline__ void mass_exchange(const Phys<R>& P, const R* qpj, R 
   if (at <= P.alphastot_min) return;
   R r_T = qpj[3];
   Mixt<R> m = mixt_var<R, NS>(P, qpj, true);
-  R inv_kin_visc = rdiv<R>(R(1), P.kin_visc_c);
   R sdep = R(0);
+  // the hindrance is that of the whole mixture: one power for all classes
+  const R hindered = P.settling ? rpow<R>(R(1) - rmin(R(1), rdiv<R>(at, alpha_max)), hind_exp) : R(0);
   for (int i = 0; i < ns; ++i) {
     if (al[i] > R(0) && P.settling) {
-      R sv = settling_velocity<R>(P, P.diam_s[i], P.rho_s[i], m.rho_c, inv_kin_visc);
+      R sv = settle ? settle[i]
+                    : settling_velocity<R>(P, P.diam_s[i], P.rho_s[i], m.rho_c, rdiv<R>(R(1), P.kin_visc_c));
       dep[i] = al[i] * sv * R(1);
-      dep[i] = dep[i] * rpow<R>(R(1) - rmin(R(1), rdiv<R>(at, alpha_max)), hind_exp);
+      dep[i] = dep[i] * hindered;
       const R cap = rdiv<R>(r_h * al[i], dt);
       if (dep_limited && !(dep[i] < cap)) *dep_limited |= 1u << i;   // the whole class settles out
       dep[i] = rmin(dep[i], cap);

@@ -286,8 +286,14 @@ class Solver : public SolverBase {
     nstat_blocks_ = 1024;
     SFLOW_CU(alloc((void**)&stat_part_, sizeof(double) * 4 * nstat_blocks_));
     SFLOW_CU(alloc((void**)&stat_out_, sizeof(double) * 4));
+    SFLOW_CU(alloc((void**)&settle_, sizeof(R) * kMaxSolid));
     SFLOW_CU(cudaMemsetAsync(q_, 0, sizeof(R) * plane_ * nv, stream_));
     fill_args();
+    if (ka_.settle) {
+      k_settling<R><<<1, 32, 0, stream_>>>(ka_.pr, settle_, hs_.ns);
+      ++launches_;
+      SFLOW_CU(cudaGetLastError());
+    }
     // shared memory of the flux kernel
     smem_flux_ = flux_smem_bytes(hs_.nv, tile_h_);
     if (!batch) SFLOW_CU(set_smem_attr());
@@ -320,7 +326,8 @@ class Solver : public SolverBase {
     if (hs_.p.bottom_radial_source_flag)
       b += A(sizeof(R) * P) + A(sizeof(double) * (1 + 2 * (size_t)SFLOW_MAX_INTERVALS));
     if (hs_.n_thk * hs_.n_dyn > 0) b += A(sizeof(uint32_t) * P * (size_t)((hs_.n_thk * hs_.n_dyn + 31) / 32));
-    b += A(sizeof(RunState)) + A(sizeof(double) * 4 * 1024) + A(sizeof(double) * 4);
+    b += A(sizeof(RunState)) + A(sizeof(double) * 4 * 1024) + A(sizeof(double) * 4) +
+         A(sizeof(R) * kMaxSolid);
     return b + extra_bytes_;
   }
   // room in the run's allocation for buffers its owner adds after init()
@@ -1013,6 +1020,7 @@ class Solver : public SolverBase {
   double* deposit_ = nullptr;
   double *erosion_ = nullptr, *erodible_ = nullptr, *Bc_ = nullptr, *bsrc_tab_ = nullptr;
   R* bfrac_ = nullptr;
+  R* settle_ = nullptr;
   uint32_t* vuln_ = nullptr;
   int vuln_words_ = 0;
   std::vector<uint8_t> tile_static_h_;   // tile_static_ on its way to the device
@@ -1445,6 +1453,7 @@ class Solver : public SolverBase {
     ka_.Bc = Bc_;
     ka_.bfrac = bfrac_;
     ka_.bsrc_tab = bsrc_tab_;
+    ka_.settle = (hs_.exchange && ka_.pr.settling && !ka_.pr.gas) ? settle_ : nullptr;
     ka_.vuln = vuln_;
     ka_.vuln_words = vuln_words_;
     ka_.take_last = hs_.take_last;
