@@ -327,7 +327,15 @@ __device__ __forceinline__ void flux_tile64(const KArgs<double>& a, const double
     const int j = j0 + cx, k = k0 + cy;
     const int rx = cx + HALO, ry = cy + HALO;
     const uint8_t fl = sfl[ry * RX + rx];
-    if (j < g.nx && k < g.ny && (fl & F_ACTIVE)) {
+    const bool active = j < g.nx && k < g.ny && (fl & F_ACTIVE);
+    if (want_dt & 2) {   // the row's active cells into the list of k_stage2_list
+      const unsigned m = __ballot_sync(0xffffffffu, active);
+      unsigned at = 0;
+      if (cx == 0 && m) at = atomicAdd(&a.st->list_n, (unsigned)__popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)__popc(m & ((1u << cx) - 1u));
+      if (active) a.cells[at] = (uint32_t)cidx(g, j, k);
+    }
+    if (active) {
       const int64_t c = cidx(g, j, k);
       if (rout) {
         double qp[np];

@@ -114,6 +114,9 @@ struct KArgs {
   const R* bfrac;    // bottom radial source: cell fraction inside the source
   const double* bsrc_tab;   // bottom radial source: n_intervals, t_intervals, vel_intervals
   const R* settle;   // settling velocities of a liquid's classes (else null)
+  // the step's active cells (k_flux64 -> k_stage2_list; FP64 single runs with
+  // N_RK = 2, else null)
+  uint32_t* cells;
   uint32_t* vuln;    // vulnerability table: words planes of 32 entries
   int vuln_words;
   RunState* st;
@@ -557,6 +560,7 @@ __global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask(KArgs<R> a
   RunState* st = a.st;
   const double t = st->t;
   if (!running(st)) return;
+  if (sizeof(R) == 8 && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) st->list_n = st->list_next = 0u;
   if ((int)blockIdx.y == tiles_y) {
     if (blockIdx.x == 0 && threadIdx.x == 0) source_factors(a, st, t);
     return;
@@ -579,6 +583,7 @@ __global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask_group(KArg
   RunState* st = a.st;
   const double t = st->t;
   if (!running(st)) return;
+  if (sizeof(R) == 8 && blockIdx.x == 0 && threadIdx.x == 0) st->list_n = st->list_next = 0u;
   const int t0 = blockIdx.x * group, ng = min(group, tiles_x * tiles_y - t0);
   if (ng <= 0) {   // the block after the last (see k_mask)
     if (threadIdx.x == 0) source_factors(a, st, t);
@@ -2073,6 +2078,43 @@ __global__ void __launch_bounds__(TX * ROWS, MIN_BLOCKS) k_stage2(KArgs<R> a, in
     } else {
       if (wet) a.tile_wet_step[(unsigned)(a.st->steps & 1) * nt + tile] = 1;
     }
+  }
+}
+
+// The fused step of the FP64 form (k_stage2's mode -1) over the list of active
+// cells that the flux kernel wrote.  Bound by the FP64 pipe and the Newton's
+// latency, so the warps want full rows of work and the SMs equal shares: by
+// 32 x 2 blocks of the grid, a flood's front (17,900 of 64,800 cells, up to 11
+// Newton iterations) ran with 11 of 32 lanes and kept one SM's FP64 pipe 88 %
+// busy where the mean was 24 %.  A warp takes 32 entries at a time: its first
+// ones spread over the SMs, the others from a counter.  Measured against those
+// blocks: 200^2 dam break 42.4 -> 31.6 us, 512^2 current 1,050 -> 998, the
+// flood 310 -> 283 (what is left is the front's own chain of Newton
+// iterations); the same bits.
+template <int NS>
+__global__ void __launch_bounds__(StageShape<double>::THREADS, StageShape<double>::MIN_BLOCKS) k_stage2_list(KArgs<double> a) {
+  step_kernel_entry();
+  RunState* st = a.st;
+  if (!st->run_step) return;
+  const unsigned n = __ldcg(&st->list_n), warps = gridDim.x * (blockDim.x / 32);
+  const int lane = threadIdx.x & 31;
+  uint8_t* wet = a.tile_wet_step + (size_t)((unsigned)st->steps & 1u) * a.g.tiles_x * a.g.tiles_y;
+  unsigned ch = threadIdx.x / 32 * gridDim.x + blockIdx.x;
+  while (ch < (n + 31u) / 32u) {
+    const unsigned i = ch * 32u + lane;
+    unsigned status = 0;
+    int nit = 0;
+    if (i < n) {
+      const unsigned c = __ldcg(a.cells + i);
+      const int k = (int)(c / (unsigned)a.g.pitch), j = (int)(c % (unsigned)a.g.pitch);
+      // wet flag of the tile for the next check_solve (see k_stage2)
+      if (stage2_cell<double, NS>(a, -1, j, k, status, nit)) wet[(k / 8) * a.g.tiles_x + j / TX] = 1;
+      if (!owned_row(a.g, k)) { status = 0u; nit = 0; }   // halo rows of a row slab
+    }
+    __syncwarp();
+    newton_stats<double>(st, status, nit, nit);
+    if (lane == 0) ch = warps + atomicAdd(&st->list_next, 1u);
+    ch = __shfl_sync(0xffffffffu, ch, 0);
   }
 }
 

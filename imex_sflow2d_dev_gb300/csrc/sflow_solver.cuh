@@ -192,7 +192,7 @@ class Solver : public SolverBase {
     SFLOW_CU(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     // one allocation for the buffers below (alloc() carves it; anything it
     // cannot hold gets its own cudaMalloc)
-    arena_cap_ = init_bytes();
+    arena_cap_ = init_bytes(batch);
     if (cudaMalloc((void**)&arena_, arena_cap_) != cudaSuccess) {
       cudaGetLastError();
       arena_ = nullptr;
@@ -287,6 +287,7 @@ class Solver : public SolverBase {
     SFLOW_CU(alloc((void**)&stat_part_, sizeof(double) * 4 * nstat_blocks_));
     SFLOW_CU(alloc((void**)&stat_out_, sizeof(double) * 4));
     SFLOW_CU(alloc((void**)&settle_, sizeof(R) * kMaxSolid));
+    if (cell_list(batch)) SFLOW_CU(alloc((void**)&cells_, sizeof(uint32_t) * plane_));
     SFLOW_CU(cudaMemsetAsync(q_, 0, sizeof(R) * plane_ * nv, stream_));
     fill_args();
     if (ka_.settle) {
@@ -307,8 +308,11 @@ class Solver : public SolverBase {
     return SFLOW_OK;
   }
 
+  // the FP64 form's N_RK = 2 step lists its active cells (a batch keeps its own)
+  bool cell_list(bool batch) const { return sizeof(R) == 8 && hs_.nrk == 2 && !batch; }
+
   // device bytes of init()'s allocations, each rounded as alloc() rounds
-  size_t init_bytes() const {
+  size_t init_bytes(bool batch) const {
     auto A = [](size_t b) { return (b + kArenaAlign - 1) / kArenaAlign * kArenaAlign; };
     const size_t P = (size_t)plane_, nv = (size_t)hs_.nv, ns = (size_t)hs_.ns;
     const size_t nstage = (hs_.nrk == 2) ? 1 : (size_t)hs_.nrk;
@@ -328,6 +332,7 @@ class Solver : public SolverBase {
     if (hs_.n_thk * hs_.n_dyn > 0) b += A(sizeof(uint32_t) * P * (size_t)((hs_.n_thk * hs_.n_dyn + 31) / 32));
     b += A(sizeof(RunState)) + A(sizeof(double) * 4 * 1024) + A(sizeof(double) * 4) +
          A(sizeof(R) * kMaxSolid);
+    if (cell_list(batch)) b += A(sizeof(uint32_t) * P);
     return b + extra_bytes_;
   }
   // room in the run's allocation for buffers its owner adds after init()
@@ -527,7 +532,7 @@ class Solver : public SolverBase {
       SFLOW_CU(cudaEventRecord(ev_[0], stream_));
       SFLOW_CU(launch_mask(2));
       SFLOW_CU(cudaEventRecord(ev_[1], stream_));
-      SFLOW_CU(launch_flux(1));
+      SFLOW_CU(launch_flux(true));
       SFLOW_CU(cudaEventRecord(ev_[2], stream_));
       SFLOW_CU(launch_step_kernel(k_dt, dim3(1), dim3(1), 0, stream_, ka_.g.pdl, st_, hs_.p.max_dt));
       ++launches_;
@@ -765,7 +770,7 @@ class Solver : public SolverBase {
   int timestep(double* dt_out) override {
     if (!uploaded_) { err_ = "no state uploaded"; return SFLOW_ESTATE; }
     if (hs_.nrk != 2) { err_ = "the per-call-site entry points need N_RK = 2; use sflow_step / sflow_advance"; return SFLOW_EINVAL; }
-    SFLOW_CU(launch_flux(1));
+    SFLOW_CU(launch_flux(false));
     RunState h;
     SFLOW_CU(cudaMemcpyAsync(&h, st_, sizeof(RunState), cudaMemcpyDeviceToHost, stream_));
     SFLOW_CU(cudaStreamSynchronize(stream_));
@@ -1021,6 +1026,7 @@ class Solver : public SolverBase {
   double *erosion_ = nullptr, *erodible_ = nullptr, *Bc_ = nullptr, *bsrc_tab_ = nullptr;
   R* bfrac_ = nullptr;
   R* settle_ = nullptr;
+  uint32_t* cells_ = nullptr;
   uint32_t* vuln_ = nullptr;
   int vuln_words_ = 0;
   std::vector<uint8_t> tile_static_h_;   // tile_static_ on its way to the device
@@ -1453,6 +1459,7 @@ class Solver : public SolverBase {
     ka_.Bc = Bc_;
     ka_.bfrac = bfrac_;
     ka_.bsrc_tab = bsrc_tab_;
+    ka_.cells = cells_;
     ka_.settle = (hs_.exchange && ka_.pr.settling && !ka_.pr.gas) ? settle_ : nullptr;
     ka_.vuln = vuln_;
     ka_.vuln_words = vuln_words_;
@@ -1500,9 +1507,10 @@ class Solver : public SolverBase {
     ++launches_;
     return tab_.mask(ka_, dim3(tiles_x_, tiles_y_), stream_, solve_all);
   }
-  cudaError_t launch_flux(int want_dt) {
+  // list: the active cells are listed for launch_stage2(-1) (FP64 form)
+  cudaError_t launch_flux(bool list) {
     ++launches_;
-    return tab_.flux(ka_, dim3(tiles_x_, tiles_y_), smem_flux_, stream_, q_, rd_, want_dt);
+    return tab_.flux(ka_, dim3(tiles_x_, tiles_y_), smem_flux_, stream_, q_, rd_, list && cells_ ? 3 : 1);
   }
   // mode -1: full fused epilogue; 0: stage only; 1: erosion only; 2: maps only
   cudaError_t launch_stage2(int mode) {
@@ -1515,7 +1523,7 @@ class Solver : public SolverBase {
     cudaError_t e;
     if (hs_.nrk == 2) {
       e = launch_mask(2);
-      if (e == cudaSuccess) e = launch_flux(1);
+      if (e == cudaSuccess) e = launch_flux(true);
       if (e == cudaSuccess) {
         e = launch_step_kernel(k_dt, dim3(1), dim3(1), 0, stream_, ka_.g.pdl, st_, hs_.p.max_dt);
         ++launches_;

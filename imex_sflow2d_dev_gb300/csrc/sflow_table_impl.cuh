@@ -171,6 +171,15 @@ static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStrea
 template <class R, int NS, int TH>
 static cudaError_t tab_stage2(const KArgs<R>& a, dim3 grid, cudaStream_t s, int mode) {
   using S = StageShape<R>;
+  if constexpr (sizeof(R) == 8) {
+    if (mode == -1) {
+      int sms = 0;
+      const cudaError_t e = sm_count(&sms);
+      if (e != cudaSuccess) return e;
+      const int64_t blocks = std::min<int64_t>((int64_t)sms * S::MIN_BLOCKS, ((int64_t)a.g.nx * a.g.ny + S::THREADS - 1) / S::THREADS);
+      return launch_step_kernel(k_stage2_list<NS>, dim3((unsigned)blocks), dim3(S::THREADS), 0, s, a.g.pdl, a);
+    }
+  }
   if constexpr (S::SMALL_ROWS != S::ROWS) {
     int sms = 0;
     const cudaError_t e = sm_count(&sms);

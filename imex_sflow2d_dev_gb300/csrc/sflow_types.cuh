@@ -98,10 +98,10 @@ struct RunState {
   long long last_cells;            // active cells of the last step
   long long newton_iters;          // sum of Newton iterations
   int newton_max;
-  int pad;
+  unsigned list_n;                 // entries in the list of active cells (FP64 single runs)
   double src_t_coeff;              // ring inlet time factor at this step's t
   float src_t_coeff_f;
-  int pad2;
+  unsigned list_next;              // next entry of it to be taken
   double tp[4];                    // time_param
   double pi_g;
   // bottom radial source at this step's t: time factor and inflow velocity
