@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, TileShape<TH>::FL
     }
     // the list holds tiles of running runs only (k_b_cand, k_b_mask)
     const int tiles_x = (a.g.nx + TX - 1) / TX;
-    flux_tile<R, NS, LIM, TH>(a, a.q, a.rd, 1, (int)(tile % (unsigned)tiles_x), (int)(tile / (unsigned)tiles_x),
+    flux_tile<R, NS, LIM, TH, true>(a, a.q, a.rd, 1, (int)(tile % (unsigned)tiles_x), (int)(tile / (unsigned)tiles_x),
                      smem_raw);
   }
 }
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kFlux64Threads, 3) k_b_flux64(BatchArgs<double
       __syncthreads();
     }
     const int tiles_x = (a.g.nx + TX - 1) / TX;
-    flux_tile64<NS, LIM>(a, a.q, a.rd, 1, (int)(tile % (unsigned)tiles_x), (int)(tile / (unsigned)tiles_x),
+    flux_tile64<NS, LIM, true>(a, a.q, a.rd, 1, (int)(tile % (unsigned)tiles_x), (int)(tile / (unsigned)tiles_x),
                          (int)(i % parts * (8u / parts)), (int)(8u / parts), smem_raw);
   }
 }

@@ -84,7 +84,7 @@ __device__ __noinline__ void recon64_other(const KArgs<double>& a, const double*
 
 // face_flux with recon64 for the ordinary cells: qf points at the divided
 // differences of this face, step to those of the next face along DIR
-template <int NS, int DIR, int LIM>
+template <int NS, int DIR, int LIM, bool FLUX>
 __device__ __forceinline__ double face_flux64(const KArgs<double>& a, const double* sqp, const uint8_t* sfl,
                                               const double* qf, int step, int sq, int f, int o, int rxl, int ryl,
                                               int rxh, int ryh, double gcs, double* H) {
@@ -148,17 +148,18 @@ __device__ __forceinline__ double face_flux64(const KArgs<double>& a, const doub
     Side<double, NS> S;
 #pragma unroll
     for (int i = 0; i < np; ++i) t[i] = s ? qph[i] : qpl[i];
-    if (s ? hh : hl) side_from_qp<double, NS, DIR>(a, t, gcs, S, s ? mirror_h : mirror_l);
+    if (s ? hh : hl) side_from_qp<double, NS, DIR, FLUX>(a, t, gcs, S, s ? mirror_h : mirror_l);
     else side_zero(S);
     if (s) Hs = S;
     else L = S;
   }
+  if constexpr (!FLUX) return rmax(rmax(rmax(L.vmax, Hs.vmax), 0.0), -rmin(rmin(L.vmin, Hs.vmin), 0.0));
   if (a.pr.scheme == SFLOW_SCHEME_UP) return up_flux<double, NS, DIR>(L, Hs, H);
   return kt_flux<double, NS, DIR>(L, Hs, H);
 }
 
 // rows r0 .. r0 + sh - 1 of tile (tx, ty)
-template <int NS, int LIM>
+template <int NS, int LIM, bool FLUX>
 __device__ __forceinline__ void flux_tile64(const KArgs<double>& a, const double* __restrict__ qin,
                                             double* __restrict__ rout, int want_dt, int tx, int ty, int r0, int sh,
                                             unsigned char* smem_raw) {
@@ -279,14 +280,16 @@ __device__ __forceinline__ void flux_tile64(const KArgs<double>& a, const double
         if (f == 0) gcs = __ldg(a.geo[5] + ch);
         else if (f == g.nx) gcs = __ldg(a.geo[5] + cl);
         else gcs = 0.5 * (__ldg(a.geo[5] + cl) + __ldg(a.geo[5] + ch));
-        amax = face_flux64<NS, 1, LIM>(a, sqp, sfl, sQx + fy * (TX + 3) + fx + 1, 1, kFlux64QX, f, k, rxl, ry, rxh, ry,
+        amax = face_flux64<NS, 1, LIM, FLUX>(a, sqp, sfl, sQx + fy * (TX + 3) + fx + 1, 1, kFlux64QX, f, k, rxl, ry, rxh, ry,
                                        gcs, H);
       } else {
 #pragma unroll
         for (int i = 0; i < nv; ++i) H[i] = 0.0;
       }
+      if constexpr (FLUX) {
 #pragma unroll
-      for (int i = 0; i < nv; ++i) sHx[i * kFlux64HX + fi] = H[i];
+        for (int i = 0; i < nv; ++i) sHx[i * kFlux64HX + fi] = H[i];
+      }
       sAx[fi] = amax;
     } else {
       const int fi = (ch - xch) * 32 + tid % 32;
@@ -307,14 +310,16 @@ __device__ __forceinline__ void flux_tile64(const KArgs<double>& a, const double
         if (f == 0) gcs = __ldg(a.geo[5] + ch);
         else if (f == g.ny) gcs = __ldg(a.geo[5] + cl);
         else gcs = 0.5 * (__ldg(a.geo[5] + cl) + __ldg(a.geo[5] + ch));
-        amax = face_flux64<NS, 2, LIM>(a, sqp, sfl, sQy + (fy + 1) * TX + fx, TX, kFlux64QY, f, j, rx, ryl, rx, ryh, gcs,
+        amax = face_flux64<NS, 2, LIM, FLUX>(a, sqp, sfl, sQy + (fy + 1) * TX + fx, TX, kFlux64QY, f, j, rx, ryl, rx, ryh, gcs,
                                        H);
       } else {
 #pragma unroll
         for (int i = 0; i < nv; ++i) H[i] = 0.0;
       }
+      if constexpr (FLUX) {
 #pragma unroll
-      for (int i = 0; i < nv; ++i) sHy[i * kFlux64HY + fi] = H[i];
+        for (int i = 0; i < nv; ++i) sHy[i * kFlux64HY + fi] = H[i];
+      }
       sAy[fi] = amax;
     }
   }
@@ -337,7 +342,7 @@ __device__ __forceinline__ void flux_tile64(const KArgs<double>& a, const double
     }
     if (active) {
       const int64_t c = cidx(g, j, k);
-      if (rout) {
+      if constexpr (FLUX) {
         double qp[np];
 #pragma unroll
         for (int i = 0; i < np; ++i) qp[i] = sqp[i * kFlux64Plane + ry * RX + rx];
@@ -398,7 +403,7 @@ __device__ __forceinline__ void flux_tile64(const KArgs<double>& a, const double
   }
 }
 
-template <int NS, int LIM>
+template <int NS, int LIM, bool FLUX>
 __global__ void __launch_bounds__(kFlux64Threads, 3)
     k_flux64(KArgs<double> a, const double* __restrict__ qin, double* __restrict__ rout, int want_dt, int sh) {
   step_kernel_entry();
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(kFlux64Threads, 3)
   const uint8_t ta = a.tile_active[ty * gridDim.x + blockIdx.x];
   const bool go = want_dt ? running(st) : st->run_step != 0;
   if (!go | (ta == 0) | (ta == TILE_DRY_BORDER)) return;
-  flux_tile64<NS, LIM>(a, qin, rout, want_dt, blockIdx.x, ty, (blockIdx.y % parts) * sh, sh, smem_raw);
+  flux_tile64<NS, LIM, FLUX>(a, qin, rout, want_dt, blockIdx.x, ty, (blockIdx.y % parts) * sh, sh, smem_raw);
 }
 
 }  // namespace sflow

@@ -862,14 +862,14 @@ struct Side {
   R un;     // upwind test of eval_flux_UP: qp u (x faces) or q hv (y faces)
 };
 
-template <class R, int NS, int DIR>
+template <class R, int NS, int DIR, bool FLUX>
 __device__ __forceinline__ void side_from_qp(const KArgs<R>& a, const R* qp, R gcs, Side<R, NS>& s,
                                              bool mirrored) {
   const Phys<R>& P = a.pr;
   Mixt<R> m = qp_to_qc_mixt<R, NS>(P, qp, s.q);
   if (mirrored) s.q[DIR] = -s.q[DIR];   // hu (x) / hv (y) of the wall mirror
   local_speeds<R, NS>(P, qp, m.red_grav, gcs, DIR, s.vmin, s.vmax);
-  eval_fluxes<R, NS>(P, s.q, qp, m, gcs, DIR, s.f);
+  if constexpr (FLUX) eval_fluxes<R, NS>(P, s.q, qp, m, gcs, DIR, s.f);
   s.hu_p = qp[1];
   s.un = (DIR == 1) ? qp[4 + NS] : s.q[2];
 }
@@ -1049,7 +1049,7 @@ __device__ __noinline__ FaceStates<R, NS> face_states_special(const KArgs<R>& a,
 // 72 registers and 3 blocks): k_flux 47.4 -> 43.1 us on a 1024^2 current, 328
 // -> 284 on a 4096^2 one, k_b_flux 58 -> 50 on an ensemble of 64 floods; the
 // same bits.
-template <class R, int NS, int DIR, int LIM, int TH>
+template <class R, int NS, int DIR, int LIM, int TH, bool FLUX>
 __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, bool plain, int f,
                                        int o, int rxl, int ryl, int rxh, int ryh, R gcs, R* H) {
   constexpr int np = 4 + NS + 2;
@@ -1068,10 +1068,11 @@ __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const ui
     flags = s.flags;
   }
   Side<R, NS> L, Hs;
-  if (flags & 1) side_from_qp<R, NS, DIR>(a, qpl, gcs, L, flags & 4);
+  if (flags & 1) side_from_qp<R, NS, DIR, FLUX>(a, qpl, gcs, L, flags & 4);
   else side_zero(L);
-  if (flags & 2) side_from_qp<R, NS, DIR>(a, qph, gcs, Hs, flags & 8);
+  if (flags & 2) side_from_qp<R, NS, DIR, FLUX>(a, qph, gcs, Hs, flags & 8);
   else side_zero(Hs);
+  if constexpr (!FLUX) return rmax(rmax(rmax(L.vmax, Hs.vmax), R(0)), -rmin(rmin(L.vmin, Hs.vmin), R(0)));
   if (a.pr.scheme == SFLOW_SCHEME_UP) return up_flux<R, NS, DIR>(L, Hs, H);
   return kt_flux<R, NS, DIR>(L, Hs, H);
 }
@@ -1084,7 +1085,12 @@ __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const ui
 // shared memory; each thread then evaluates one face (both reconstructed
 // sides, speeds, physical fluxes, KT flux) and finally one cell.
 // ---------------------------------------------------------------------------
-template <class R, int NS, int LIM, int TH>
+// FLUX = false: the CFL minimum alone (the timestep pass of a tableau whose
+// first stage takes no flux): no physical fluxes, no explicit terms.  Its own
+// instantiation: 401 x 263 dam break, N_RK = 3, 91 -> 85 us a step, against 89
+// with the same kernel testing rout, which also cost the batch (50 -> 60 us a
+// launch on an ensemble of 64 floods) its registers.
+template <class R, int NS, int LIM, int TH, bool FLUX>
 __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict__ qin,
                                           R* __restrict__ rout, int want_dt, int tx, int ty,
                                           unsigned char* smem_raw) {
@@ -1214,13 +1220,15 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
       if (!plain && f == 0) gcs = __ldg(a.geo[5] + ch);
       else if (!plain && f == g.nx) gcs = __ldg(a.geo[5] + cl);
       else gcs = cst<R>(0.5) * (__ldg(a.geo[5] + cl) + __ldg(a.geo[5] + ch));
-      amax = face_flux<R, NS, 1, LIM, TH>(a, sqp, sfl, plain, f, k, rxl, ry, rxh, ry, gcs, H);
+      amax = face_flux<R, NS, 1, LIM, TH, FLUX>(a, sqp, sfl, plain, f, k, rxl, ry, rxh, ry, gcs, H);
     } else {
 #pragma unroll
       for (int i = 0; i < nv; ++i) H[i] = R(0);
     }
+    if constexpr (FLUX) {
 #pragma unroll
-    for (int i = 0; i < nv; ++i) sHx[i * TY * (TX + 1) + fi] = H[i];
+      for (int i = 0; i < nv; ++i) sHx[i * TY * (TX + 1) + fi] = H[i];
+    }
     sAx[fi] = amax;
   }
 
@@ -1245,13 +1253,15 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
       if (!plain && f == 0) gcs = __ldg(a.geo[5] + ch);
       else if (!plain && f == g.ny) gcs = __ldg(a.geo[5] + cl);
       else gcs = cst<R>(0.5) * (__ldg(a.geo[5] + cl) + __ldg(a.geo[5] + ch));
-      amax = face_flux<R, NS, 2, LIM, TH>(a, sqp, sfl, plain, f, j, rx, ryl, rx, ryh, gcs, H);
+      amax = face_flux<R, NS, 2, LIM, TH, FLUX>(a, sqp, sfl, plain, f, j, rx, ryl, rx, ryh, gcs, H);
     } else {
 #pragma unroll
       for (int i = 0; i < nv; ++i) H[i] = R(0);
     }
+    if constexpr (FLUX) {
 #pragma unroll
-    for (int i = 0; i < nv; ++i) sHy[i * (TY + 1) * TX + fi] = H[i];
+      for (int i = 0; i < nv; ++i) sHy[i * (TY + 1) * TX + fi] = H[i];
+    }
     sAy[fi] = amax;
   }
   __syncthreads();
@@ -1267,45 +1277,47 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
     const int rx = cx + HALO, ry = cy + HALO;
     if (j < g.nx && k < g.ny && (sfl[ry * RX + rx] & F_ACTIVE)) {
       const int64_t c = cidx(g, j, k);
-      R qp[np];
+      if constexpr (FLUX) {
+        R qp[np];
 #pragma unroll
-      for (int i = 0; i < np; ++i) qp[i] = sqp[i * RX * RY + ry * RX + rx];
-      R e[nv];
-      Geo<R> geo;   // this thread's copies of step 0
-      geo.Bx = sgeo[tid];
-      geo.By = sgeo[TX * TY + tid];
-      geo.gc = sgeo[2 * TX * TY + tid];
-      geo.dgcx = sgeo[3 * TX * TY + tid];
-      geo.dgcy = sgeo[4 * TX * TY + tid];
-      geo.Bxx = a.geo[2] ? __ldg(a.geo[2] + c) : R(0);
-      geo.Bxy = a.geo[3] ? __ldg(a.geo[3] + c) : R(0);
-      geo.Byy = a.geo[4] ? __ldg(a.geo[4] + c) : R(0);
-      const uint8_t fl = sfl[ry * RX + rx];
-      R ap = R(0), anx = R(0), any_ = R(0);
-      R tcoef = R(0);   // read at ring cells only (arc perimeter > 0)
-      if (P.radial_source && (fl & F_SC_MASK) == 2) {
-        ap = __ldg(a.arc + c);
-        anx = __ldg(a.arc + g.plane + c);
-        any_ = __ldg(a.arc + 2 * g.plane + c);
-        if constexpr (sizeof(R) == 8) tcoef = st->src_t_coeff;
-        else tcoef = st->src_t_coeff_f;
-      }
-      R bf = R(0), btc = R(0), bvel = R(0);   // bottom source cells only
-      if (P.bottom_source && any_bsrc_tile && (__ldg(a.cflags + c) & F_BSRC)) {
-        bf = __ldg(a.bfrac + c);
-        if constexpr (sizeof(R) == 8) { btc = st->bsrc_t_coeff; bvel = st->bsrc_vel; }
-        else { btc = st->bsrc_t_coeff_f; bvel = st->bsrc_vel_f; }
-      }
-      expl_terms<R, NS>(P, geo, qp, tcoef, ap, anx, any_, bf, btc, bvel, e);
-#pragma unroll
-      for (int i = 0; i < nv; ++i) {
-        R d = R(0);
-        if (!tile_dry) {
-          d = d + (sHx[i * TY * (TX + 1) + cy * (TX + 1) + cx + 1] - sHx[i * TY * (TX + 1) + cy * (TX + 1) + cx]) * g.one_by_dx;
-          if (g.ny > 1)
-            d = d + (sHy[i * (TY + 1) * TX + (cy + 1) * TX + cx] - sHy[i * (TY + 1) * TX + cy * TX + cx]) * g.one_by_dy;
+        for (int i = 0; i < np; ++i) qp[i] = sqp[i * RX * RY + ry * RX + rx];
+        R e[nv];
+        Geo<R> geo;   // this thread's copies of step 0
+        geo.Bx = sgeo[tid];
+        geo.By = sgeo[TX * TY + tid];
+        geo.gc = sgeo[2 * TX * TY + tid];
+        geo.dgcx = sgeo[3 * TX * TY + tid];
+        geo.dgcy = sgeo[4 * TX * TY + tid];
+        geo.Bxx = a.geo[2] ? __ldg(a.geo[2] + c) : R(0);
+        geo.Bxy = a.geo[3] ? __ldg(a.geo[3] + c) : R(0);
+        geo.Byy = a.geo[4] ? __ldg(a.geo[4] + c) : R(0);
+        const uint8_t fl = sfl[ry * RX + rx];
+        R ap = R(0), anx = R(0), any_ = R(0);
+        R tcoef = R(0);   // read at ring cells only (arc perimeter > 0)
+        if (P.radial_source && (fl & F_SC_MASK) == 2) {
+          ap = __ldg(a.arc + c);
+          anx = __ldg(a.arc + g.plane + c);
+          any_ = __ldg(a.arc + 2 * g.plane + c);
+          if constexpr (sizeof(R) == 8) tcoef = st->src_t_coeff;
+          else tcoef = st->src_t_coeff_f;
         }
-        if (rout) rout[i * g.plane + c] = d - e[i];
+        R bf = R(0), btc = R(0), bvel = R(0);   // bottom source cells only
+        if (P.bottom_source && any_bsrc_tile && (__ldg(a.cflags + c) & F_BSRC)) {
+          bf = __ldg(a.bfrac + c);
+          if constexpr (sizeof(R) == 8) { btc = st->bsrc_t_coeff; bvel = st->bsrc_vel; }
+          else { btc = st->bsrc_t_coeff_f; bvel = st->bsrc_vel_f; }
+        }
+        expl_terms<R, NS>(P, geo, qp, tcoef, ap, anx, any_, bf, btc, bvel, e);
+#pragma unroll
+        for (int i = 0; i < nv; ++i) {
+          R d = R(0);
+          if (!tile_dry) {
+            d = d + (sHx[i * TY * (TX + 1) + cy * (TX + 1) + cx + 1] - sHx[i * TY * (TX + 1) + cy * (TX + 1) + cx]) * g.one_by_dx;
+            if (g.ny > 1)
+              d = d + (sHy[i * (TY + 1) * TX + (cy + 1) * TX + cx] - sHy[i * (TY + 1) * TX + cy * TX + cx]) * g.one_by_dy;
+          }
+          rout[i * g.plane + c] = d - e[i];
+        }
       }
       if (want_dt && !tile_dry && owned_row(g, k)) {
         R ax = rmax(sAx[cy * (TX + 1) + cx], sAx[cy * (TX + 1) + cx + 1]);
@@ -1392,7 +1404,7 @@ static __global__ void k_dt(RunState* st, double max_dt) {
   dt_update(st, max_dt);
 }
 
-template <class R, int NS, int LIM, int TH>
+template <class R, int NS, int LIM, int TH, bool FLUX>
 __global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, LIM == 1 ? TileShape<TH>::FLUX_MIN_BLOCKS : 1)
     k_flux(KArgs<R> a, const R* __restrict__ qin, R* __restrict__ rout, int want_dt) {
   step_kernel_entry();
@@ -1403,7 +1415,7 @@ __global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, LIM == 1 ? TileSh
   const uint8_t ta = a.tile_active[blockIdx.y * gridDim.x + blockIdx.x];
   const bool go = want_dt ? running(st) : st->run_step != 0;
   if (!go | (ta == 0) | (ta == TILE_DRY_BORDER)) return;
-  flux_tile<R, NS, LIM, TH>(a, qin, rout, want_dt, blockIdx.x, blockIdx.y, smem_raw);
+  flux_tile<R, NS, LIM, TH, FLUX>(a, qin, rout, want_dt, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // ---------------------------------------------------------------------------

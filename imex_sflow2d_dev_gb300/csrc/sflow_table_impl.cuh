@@ -148,24 +148,28 @@ static cudaError_t tab_mask(const KArgs<R>& a, dim3 grid, cudaStream_t s, int so
   return launch_step_kernel(k_mask_group<R, TH>, dim3((unsigned)((tiles + group - 1) / group) + src), T, 0, s, a.g.pdl,
                             a, tx, ty, group);
 }
+// minmod everywhere (the reference default) has its own instantiation: one
+// limiter case instead of eight per variable keeps the code small.  So does the
+// pass without fluxes (rout null).
+template <class R, int NS, int TH, bool FLUX>
+static auto flux_kernel(bool minmod) {
+  if constexpr (sizeof(R) == 8) return minmod ? &k_flux64<NS, 1, FLUX> : &k_flux64<NS, -1, FLUX>;
+  else return minmod ? &k_flux<R, NS, 1, TH, FLUX> : &k_flux<R, NS, -1, TH, FLUX>;
+}
 template <class R, int NS, int TH>
 static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStream_t s, const R* qin,
                             R* rout, int want_dt) {
-  // minmod everywhere (the reference default) has its own instantiation:
-  // one limiter case instead of eight per variable keeps the code small
+  const bool minmod = a.g.lim_all == 1;
+  const auto kern = rout ? flux_kernel<R, NS, TH, true>(minmod) : flux_kernel<R, NS, TH, false>(minmod);
   if constexpr (sizeof(R) == 8) {
     int sms = 0;
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
     const int sh = flux64_rows((int64_t)grid.x * grid.y, sms);
     grid.y *= 8 / sh;
-    const dim3 T(kFlux64Threads);
-    if (a.g.lim_all == 1) return launch_step_kernel(k_flux64<NS, 1>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt, sh);
-    return launch_step_kernel(k_flux64<NS, -1>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt, sh);
+    return launch_step_kernel(kern, grid, dim3(kFlux64Threads), smem, s, a.g.pdl, a, qin, rout, want_dt, sh);
   } else {
-    const dim3 T(TileShape<TH>::FLUX_THREADS);
-    if (a.g.lim_all == 1) return launch_step_kernel(k_flux<R, NS, 1, TH>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt);
-    return launch_step_kernel(k_flux<R, NS, -1, TH>, grid, T, smem, s, a.g.pdl, a, qin, rout, want_dt);
+    return launch_step_kernel(kern, grid, dim3(TileShape<TH>::FLUX_THREADS), smem, s, a.g.pdl, a, qin, rout, want_dt);
   }
 }
 template <class R, int NS, int TH>
@@ -204,15 +208,13 @@ static cudaError_t tab_assemble(const KArgs<R>& a, dim3 grid, cudaStream_t s) {
 }
 template <class R, int NS, int TH>
 static cudaError_t tab_smem(size_t bytes) {
-  if constexpr (sizeof(R) == 8) {
-    cudaError_t e = cudaFuncSetAttribute(k_flux64<NS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  for (int minmod = 0; minmod < 2; ++minmod) {
+    cudaError_t e = cudaFuncSetAttribute(flux_kernel<R, NS, TH, true>(minmod), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(flux_kernel<R, NS, TH, false>(minmod), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_flux64<NS, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  } else {
-    cudaError_t e = cudaFuncSetAttribute(k_flux<R, NS, 1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_flux<R, NS, -1, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   }
+  return cudaSuccess;
 }
 // the batched flux kernel of a form and its threads
 template <class R, int NS, int LIM, int TH>
