@@ -438,20 +438,21 @@ __global__ void __launch_bounds__(kBatchStageThreads<R>, 4) k_b_stage2(BatchArgs
     const unsigned grp = __match_any_sync(0xffffffffu, slot);
     const int leader = __ffs(grp) - 1;
     int sum = 0, mx = 0;
-    unsigned st_or = 0;
-    for (unsigned m = grp; m; m &= m - 1u) {
-      const int src = __ffs(m) - 1;
-      sum += __shfl_sync(grp, nit, src);
-      mx = max(mx, __shfl_sync(grp, nit, src));
-      st_or |= __shfl_sync(grp, status, src);
-    }
-    if (lane == leader && slot >= 0) {
-      RunState* st = b.args[slot].st;
-      if (st_or) atomicOr(&st->status, st_or);
-      if (sum > 0) {
-        atomicAdd((unsigned long long*)&st->newton_iters, (unsigned long long)sum);
-        atomicMax(&st->newton_max, mx);
+    if (grp == 0xffffffffu) {   // the whole warp in one run: almost always
+      sum = __reduce_add_sync(0xffffffffu, nit);
+      mx = __reduce_max_sync(0xffffffffu, nit);
+    } else {
+      for (unsigned m = grp; m; m &= m - 1u) {
+        const int src = __ffs(m) - 1;
+        const int v = __shfl_sync(grp, nit, src);
+        sum += v;
+        mx = max(mx, v);
       }
+    }
+    if (slot >= 0) {
+      RunState* st = b.args[slot].st;
+      if (status) atomicOr(&st->status, status);
+      if (lane == leader) newton_add(st, sum, mx);
     }
   }
 }
