@@ -1981,7 +1981,9 @@ __device__ __forceinline__ unsigned stage_cell(const KArgs<R>& a, const Geo<R>& 
 
 // A step's Newton counters: every warp or block adds to the same two words, so
 // the maximum is only sent when it is one (with that and one addition per block
-// instead of per warp, k_stage2 of a 1024^2 FP32 current 30.7 -> 29.0 us).
+// instead of per warp, k_stage2 of a 1024^2 FP32 current 30.7 -> 29.0 us;
+// warps that add for themselves in a small domain's 4-row blocks: 517 x 333
+// collapse 14.3 -> 16.2).
 __device__ __forceinline__ void newton_add(RunState* st, int sum, int mx) {
   if (sum > 0) {
     atomicAdd((unsigned long long*)&st->newton_iters, (unsigned long long)sum);
@@ -2004,6 +2006,11 @@ __device__ __forceinline__ void newton_stats(RunState* st, unsigned status, int 
 // 0: stage + assembly (imex_RK_solver); 1: erosion/deposition only;
 // 2: maxima only.
 // ---------------------------------------------------------------------------
+// The planes read only at the end of the cell's chain start on their way when
+// it starts: 4096^2 current with deposits 529 -> 522 us, no change where the
+// state fits L2.
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // One cell (j, k) of the pointwise step; returns 1 when the cell is active
 // and holds mass afterwards.  One cell per thread in every caller, so the
 // cell's arithmetic is the same code whatever the tile height.
@@ -2030,6 +2037,15 @@ __device__ __forceinline__ int stage2_cell(const KArgs<R>& a, int mode, int j, i
       post_step_maps<R, NS>(a, c, q);
     }
   } else {
+    if (mode < 0) {
+      prefetch_l1(a.hmax + c);
+      prefetch_l1(a.pdynmax + c);
+      prefetch_l1(a.mvmax + c);
+      if (a.deposit) {
+#pragma unroll
+        for (int i = 0; i < NS; ++i) prefetch_l1(a.deposit + i * g.plane + c);
+      }
+    }
     const Geo<R> geo = load_geo(a, c);
     R s1[nv], s2[nv], rn[nv];
 #pragma unroll
