@@ -1094,6 +1094,7 @@ template <class R, int NS, int LIM, int TH, bool FLUX>
 __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict__ qin,
                                           R* __restrict__ rout, int want_dt, int tx, int ty,
                                           unsigned char* smem_raw) {
+  static_assert(sizeof(R) == 4, "the FP64 form has flux_tile64");
   constexpr int TY = TH, RY = TileShape<TH>::RY, FLUX_THREADS = TileShape<TH>::FLUX_THREADS;
   constexpr int nv = 4 + NS, np = nv + 2;
   const RunState* st = a.st;
@@ -1122,10 +1123,7 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
 #pragma unroll
       for (int p = 0; p < 5; ++p) {
         const unsigned dst = (unsigned)__cvta_generic_to_shared(sgeo + p * TX * TY + tid);
-        if constexpr (sizeof(R) == 4)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src[p]) : "memory");
-        else
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src[p]) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src[p]) : "memory");
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -1298,14 +1296,13 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
           ap = __ldg(a.arc + c);
           anx = __ldg(a.arc + g.plane + c);
           any_ = __ldg(a.arc + 2 * g.plane + c);
-          if constexpr (sizeof(R) == 8) tcoef = st->src_t_coeff;
-          else tcoef = st->src_t_coeff_f;
+          tcoef = st->src_t_coeff_f;
         }
         R bf = R(0), btc = R(0), bvel = R(0);   // bottom source cells only
         if (P.bottom_source && any_bsrc_tile && (__ldg(a.cflags + c) & F_BSRC)) {
           bf = __ldg(a.bfrac + c);
-          if constexpr (sizeof(R) == 8) { btc = st->bsrc_t_coeff; bvel = st->bsrc_vel; }
-          else { btc = st->bsrc_t_coeff_f; bvel = st->bsrc_vel_f; }
+          btc = st->bsrc_t_coeff_f;
+          bvel = st->bsrc_vel_f;
         }
         expl_terms<R, NS>(P, geo, qp, tcoef, ap, anx, any_, bf, btc, bvel, e);
 #pragma unroll
@@ -1322,15 +1319,9 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
       if (want_dt && !tile_dry && owned_row(g, k)) {
         R ax = rmax(sAx[cy * (TX + 1) + cx], sAx[cy * (TX + 1) + cx + 1]);
         R ay = (g.ny > 1) ? rmax(sAy[cy * TX + cx], sAy[(cy + 1) * TX + cx]) : R(0);
-        if constexpr (sizeof(R) == 8) {
-          double dtx = (ax > 0.0) ? ddiv64(g.cfl * g.dx, ax) : 1.0e300;
-          double dty = (ay > 0.0) ? ddiv64(g.cfl * g.dy, ay) : 1.0e300;
-          dtloc = rmin(dtx, dty);
-        } else {
-          float dtx = (ax > 0.0f) ? fdiv(g.cfl_dx, ax) : 3.0e38f;
-          float dty = (ay > 0.0f) ? fdiv(g.cfl_dy, ay) : 3.0e38f;
-          dtloc = fminf(dtx, dty);
-        }
+        float dtx = (ax > 0.0f) ? fdiv(g.cfl_dx, ax) : 3.0e38f;
+        float dty = (ay > 0.0f) ? fdiv(g.cfl_dy, ay) : 3.0e38f;
+        dtloc = fminf(dtx, dty);
       }
     }
   }
@@ -1345,7 +1336,7 @@ __device__ __forceinline__ void flux_tile(const KArgs<R>& a, const R* __restrict
       R b = wmin[0];
       for (int w = 1; w < FLUX_THREADS / 32; ++w) b = rmin(b, wmin[w]);
       const double bd = (double)b;
-      if (bd < (sizeof(R) == 8 ? 1.0e300 : 3.0e38)) atomicMin(&a.st->dtmin_bits, dbits(bd));
+      if (bd < 3.0e38) atomicMin(&a.st->dtmin_bits, dbits(bd));
     }
   }
 }
@@ -2109,7 +2100,7 @@ __global__ void __launch_bounds__(TX * ROWS, MIN_BLOCKS) k_stage2(KArgs<R> a, in
     for (int r = 0; r < ROWS; ++r) { sum += s_sum[r]; mx = max(mx, s_max[r]); }
     newton_add(a.st, sum, mx);
   }
-  if (mode < 0) {
+  if (sizeof(R) == 4 && mode < 0) {   // FP64: k_stage2_list
     // wet flag of the tile for the next check_solve (buffer of the new
     // step count's parity; set only, the check_solve of this step cleared it)
     const int nt = gridDim.x * a.g.tiles_y;

@@ -806,14 +806,6 @@ __device__ __forceinline__ void mass_exchange(const Phys<R>& P, const R* qpj, R 
 // one FP64 Newton step with the analytic derivative finishes it.
 // ---------------------------------------------------------------------------
 
-// 1/x to ~1 ulp: float estimate + two Newton-Raphson refinements in FP64
-__device__ __forceinline__ double rcp64(double x) {
-  double r = (double)__frcp_rn((float)x);
-  r = r * (2.0 - x * r);
-  r = r * (2.0 - x * r);
-  return r;
-}
-
 // The same root with every coefficient formed in FP64 from the FP32 state
 // (entering through f2d_exact) and Newton iterated in FP64 with its FP64
 // derivative to a relative step of 4 ulp (the reference's TOLX is the
