@@ -61,7 +61,9 @@ constexpr int kTileHDefault = 8;
 //        so small blocks spread over the SMs best; held to 168 registers for
 //        12 warps per SM its spills cost more than the warps gave (512^2
 //        current 1.04 against 1.14 ms, eroding flood 0.36 against 0.39; 8
-//        rows, 1 block: 1.05 and 0.42).
+//        rows, 1 block: 1.05 and 0.42).  (Measured by rows of the grid, as the
+//        per-call-site entries run; the fused step's k_stage2_list has blocks
+//        of the same size.)
 template <class R>
 struct StageShape {
   static constexpr int ROWS = sizeof(R) == 4 ? 8 : 2;
@@ -1055,7 +1057,15 @@ __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const ui
   constexpr int np = 4 + NS + 2;
   R qpl[np], qph[np];
   int flags = 3;
-  if (plain) {
+  // in a special tile the faces away from the edge and the ring are ordinary too
+  // (a batch of 256 ring-inlet runs, whose tiles are mostly special: 112.4 ->
+  // 111.3 us a launch)
+  const int n = (DIR == 1) ? a.g.nx : a.g.ny;
+  bool ordinary = plain;
+  if (!plain && f > 1 && f < n - 1) {
+    ordinary = !(a.pr.radial_source && ((sfl[ryl * RX + rxl] | sfl[ryh * RX + rxh]) & F_SC_MASK));
+  }
+  if (ordinary) {
     recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxl, ryl, f - 1, 1, qpl);
     recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxh, ryh, f, 0, qph);
   } else {
@@ -1999,13 +2009,14 @@ __device__ __forceinline__ void newton_stats(RunState* st, unsigned status, int 
 // ---------------------------------------------------------------------------
 // The planes read only at the end of the cell's chain start on their way when
 // it starts: 4096^2 current with deposits 529 -> 522 us, no change where the
-// state fits L2.
+// state fits L2.  Not in a batch, whose cells are scattered (256 ring-inlet
+// runs: 33.3 us a launch without, 34.6 with).
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 // One cell (j, k) of the pointwise step; returns 1 when the cell is active
 // and holds mass afterwards.  One cell per thread in every caller, so the
 // cell's arithmetic is the same code whatever the tile height.
-template <class R, int NS>
+template <class R, int NS, bool PREFETCH = false>
 __device__ __forceinline__ int stage2_cell(const KArgs<R>& a, int mode, int j, int k, unsigned& status,
                                            int& nit) {
   constexpr int nv = 4 + NS;
@@ -2028,7 +2039,7 @@ __device__ __forceinline__ int stage2_cell(const KArgs<R>& a, int mode, int j, i
       post_step_maps<R, NS>(a, c, q);
     }
   } else {
-    if (mode < 0) {
+    if (PREFETCH && mode < 0) {
       prefetch_l1(a.hmax + c);
       prefetch_l1(a.pdynmax + c);
       prefetch_l1(a.mvmax + c);
@@ -2087,7 +2098,7 @@ __global__ void __launch_bounds__(TX * ROWS, MIN_BLOCKS) k_stage2(KArgs<R> a, in
   }
   unsigned status = 0;
   int nit = 0;
-  const int wet = run ? stage2_cell<R, NS>(a, mode, blockIdx.x * TX + threadIdx.x % TX, kk, status, nit) : 0;
+  const int wet = run ? stage2_cell<R, NS, true>(a, mode, blockIdx.x * TX + threadIdx.x % TX, kk, status, nit) : 0;
   if (!owned_row(a.g, kk)) { status = 0u; nit = 0; }   // halo rows of a row slab
   if (status) atomicOr(&a.st->status, status);
   __shared__ int s_sum[ROWS], s_max[ROWS];
