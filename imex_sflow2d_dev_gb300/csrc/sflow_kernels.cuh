@@ -991,7 +991,7 @@ struct FaceStates {
   int flags;
 };
 template <class R, int NS, int DIR, int LIM, int TH>
-__device__ __noinline__ FaceStates<R, NS> face_states_special(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f,
+__device__ __forceinline__ FaceStates<R, NS> face_states_special(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f,
                                                               int o, int rxl, int ryl, int rxh, int ryh) {
   constexpr int nv = 4 + NS, np = nv + 2;
   constexpr int vel = (DIR == 1) ? nv : nv + 1;
@@ -1046,11 +1046,13 @@ __device__ __noinline__ FaceStates<R, NS> face_states_special(const KArgs<R>& a,
 // the dry one that an absent side has.)
 // The kernel is bound by instructions, two thirds of them not arithmetic; the
 // special faces' rules and their states in local memory were part of it for
-// every face.  With them out of line and passed by value, and 4 blocks per SM
-// (56 registers, a few spills; the generic-limiter kernel is faster with its
-// 72 registers and 3 blocks): k_flux 47.4 -> 43.1 us on a 1024^2 current, 328
-// -> 284 on a 4096^2 one, k_b_flux 58 -> 50 on an ensemble of 64 floods; the
-// same bits.
+// every face.  With them on a path of their own, the cells' edge rules by value
+// out of line, and 4 blocks per SM (56 registers, a few spills; the
+// generic-limiter kernel is faster with its 72 registers and 3 blocks): k_flux
+// 47.4 -> 40.6 us on a 1024^2 current, 328 -> 264 on a 4096^2 one, k_b_flux 58
+// -> 48 on a batch of 64 floods.  A batch of 256 ring-inlet runs, most of whose
+// tiles are special: 99 -> 106 (111 with the whole special path out of line),
+// made up by check_solve; the same bits.
 template <class R, int NS, int DIR, int LIM, int TH, bool FLUX>
 __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, bool plain, int f,
                                        int o, int rxl, int ryl, int rxh, int ryh, R gcs, R* H) {
