@@ -259,14 +259,32 @@ __device__ __forceinline__ long long newton_maxf(const double* f) {
   return m;
 }
 
+// The closure as solve_rk_step reads it (a host test of the iteration passes
+// one of its own).
+template <int NS>
+struct Friction {
+  static __device__ __forceinline__ void real(const Phys<double>& P, double Bx, double By, const Div64& dxi,
+                                              const double* q, FrictPoint& f, double& nh1, double& nh2) {
+    friction_real<NS>(P, Bx, By, dxi, q, f, nh1, nh2);
+  }
+  static __device__ __forceinline__ void imag(const Phys<double>& P, double Bx, double By, const Div64& dxi,
+                                              const FrictPoint& f, int col, double q1, double q2, double q3, double e,
+                                              double& im1, double& im2) {
+    friction_imag(P, Bx, By, dxi, f, col, q1, q2, q3, e, im1, im2);
+  }
+};
+
 // solve_rk_step (normalize_q = T, normalize_f = F, opt_search_NL = T;
 // implicit set {hu, hv}); returns the iterations used (kMaxNewton + 1 when
 // the limit was reached).  The line search's cubic model never chooses its
 // step: its minimiser is capped at half the last step and the step kept above
 // the same half (solver_2d.f90:2205-2222), so after the first refusal, which
-// follows the quadratic model, the step is halved.  One loop evaluates the closure for every purpose, so that the
-// code holds it once (the kernel's code exceeds the instruction cache).
-template <int NS>
+// follows the quadratic model, the step is halved.  The quadratic model's own
+// step may be infinite or return to 1, and then no halving reaches the least
+// step: after kMaxTrials refusals the last trial is taken, which bounds the
+// search.  One loop evaluates the closure for every purpose, so that the code
+// holds it once (the kernel's code exceeds the instruction cache).
+template <int NS, class F = Friction<NS>>
 __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
   constexpr int nv = 4 + NS;
   const double STPMX = 100.0, TOLF = 1.0e-10, TOLX = kEps;
@@ -280,10 +298,10 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
 #pragma unroll
   for (int i = 0; i < nv; ++i) dtR[i] = c.dt * c.Rj[i];
   enum { START, SCALED, FIRST, TRIAL } phase = START;
-  int it = 0;
+  int it = 0, trials = 0;
 #pragma unroll 1
   for (;;) {
-    friction_real<NS>(P, c.Bx, c.By, dxi, qj, fp, nh1, nh2);
+    F::real(P, c.Bx, c.By, dxi, qj, fp, nh1, nh2);
     if (phase != SCALED) newton_residual<NS>(c, dtR, qj, nh1, nh2, f, scal_f);
     if (phase == START) {
       if (newton_maxf<NS>(f) < d64_bits(TOLF)) return 1;
@@ -316,15 +334,17 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
           alamin = ddiv64(TOLX, mx);
         }
         const bool stop = alam < alamin;
-        const double quad = (alam == 1.0) ? -slope / (2.0 * (scal_f - scal_old - slope)) : 0.0;
-        alam = (quad > 0.5 * alam) ? quad : 0.5 * alam;
+        if (stop || ++trials < kMaxTrials) {
+          const double quad = (alam == 1.0) ? -slope / (2.0 * (scal_f - scal_old - slope)) : 0.0;
+          alam = (quad > 0.5 * alam) ? quad : 0.5 * alam;
 #pragma unroll
-        for (int i = 0; i < nv; ++i) {
-          rel[i] = stop ? xo[i] : xo[i] + alam * p[i];
-          qj[i] = rel[i] * org[i];
+          for (int i = 0; i < nv; ++i) {
+            rel[i] = stop ? xo[i] : xo[i] + alam * p[i];
+            qj[i] = rel[i] * org[i];
+          }
+          if (stop) return it;
+          continue;
         }
-        if (stop) return it;
-        continue;
       }
       if (newton_maxf<NS>(f) < d64_bits(TOLF)) return it;
       // |step| < TOLX max(|rel|, 1) in every component: TOLX is a power of
@@ -349,7 +369,7 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
 #pragma unroll 1
     for (int col = 0; col < 2; ++col) {
       double a1, a2;
-      friction_imag(P, c.Bx, c.By, dxi, fp, col, qj[1], qj[2], qj[3], h * (col ? org[2] : org[1]), a1, a2);
+      F::imag(P, c.Bx, c.By, dxi, fp, col, qj[1], qj[2], qj[3], h * (col ? org[2] : org[1]), a1, a2);
       if (col) { j1[1] = a1; j2[1] = a2; }
       else { j1[0] = a1; j2[0] = a2; }
     }
@@ -370,6 +390,7 @@ __device__ __forceinline__ int solve_rk_step(const NewtonCtx& c, double* qj) {
     phase = (it == 1) ? FIRST : TRIAL;
     if (it > 1) {
       alam = 1.0;
+      trials = 0;
       slope = 0.0;
       alamin = -1.0;
       if (!d64_lt(nrm, (99.0 * nv) * (99.0 * nv))) {

@@ -9,6 +9,7 @@ namespace sflow {
 constexpr int kMaxSolid = SFLOW_MAX_SOLID;
 constexpr int kMaxVars = SFLOW_MAX_VARS;   // conservative variables
 constexpr int kMaxNewton = 100;            // max_nl_iter (parameters_2d.f90:362)
+constexpr int kMaxTrials = 4096;           // trials of one line search (FP64 form)
 
 // Physical constants and model flags, in the bulk arithmetic type R.  A
 // double copy always exists for the FP64 parts (Newton, epilogue).
