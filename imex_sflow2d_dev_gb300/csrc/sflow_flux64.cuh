@@ -410,11 +410,12 @@ __global__ void __launch_bounds__(kFlux64Threads, 3)
   const RunState* st = a.st;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // see k_flux
-  const int parts = 8 / sh, ty = blockIdx.y / parts;
+  const int parts = 8 / sh, by = block_row(), ty = by / parts;
+  if (ty >= a.g.tiles_y) return;
   const uint8_t ta = a.tile_active[ty * gridDim.x + blockIdx.x];
   const bool go = want_dt ? running(st) : st->run_step != 0;
   if (!go | (ta == 0) | (ta == TILE_DRY_BORDER)) return;
-  flux_tile64<NS, LIM, FLUX>(a, qin, rout, want_dt, blockIdx.x, ty, (blockIdx.y % parts) * sh, sh, smem_raw);
+  flux_tile64<NS, LIM, FLUX>(a, qin, rout, want_dt, blockIdx.x, ty, (by % parts) * sh, sh, smem_raw);
 }
 
 }  // namespace sflow

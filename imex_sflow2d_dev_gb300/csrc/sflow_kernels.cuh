@@ -146,6 +146,23 @@ static cudaError_t launch_step_kernel(void (*kern)(KParams...), dim3 grid, dim3 
   cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
+// A grid of `rows` block rows over tiles.y tile rows.  More than grid.y's
+// 65,535 (a tall FP64 domain, whose blocks are parts of a tile; the block of
+// k_mask after the last tile) are folded over grid.z, and the kernel's row is
+// block_row(), which may lie past the last one then.  Domains of more than
+// 65,535 tile rows stay refused by the launch.
+static inline dim3 row_grid(dim3 tiles, unsigned rows) {
+  const unsigned z = tiles.y > 65535u ? 1u : (rows + 65534u) / 65535u;
+  return dim3(tiles.x, (rows + z - 1u) / z, z);
+}
+__device__ __forceinline__ int block_row() { return (int)(blockIdx.z * gridDim.y + blockIdx.y); }
+// of the pointwise kernels: FP32 blocks hold at least a tile's rows or eight,
+// so theirs are never folded
+template <class R>
+__device__ __forceinline__ int stage_row() {
+  return sizeof(R) == 8 ? block_row() : (int)blockIdx.y;
+}
+
 template <class R>
 __device__ __forceinline__ int64_t cidx(const Grid<R>& g, int j, int k) {
   return (int64_t)k * g.pitch + j;
@@ -562,13 +579,14 @@ __global__ void __launch_bounds__(TileShape<TH>::MASK_THREADS) k_mask(KArgs<R> a
   RunState* st = a.st;
   const double t = st->t;
   if (!running(st)) return;
-  if (sizeof(R) == 8 && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) st->list_n = st->list_next = 0u;
-  if ((int)blockIdx.y == tiles_y) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) source_factors(a, st, t);
+  const int ty = block_row();
+  if (sizeof(R) == 8 && blockIdx.x == 0 && ty == 0 && threadIdx.x == 0) st->list_n = st->list_next = 0u;
+  if (ty >= tiles_y) {
+    if (ty == tiles_y && blockIdx.x == 0 && threadIdx.x == 0) source_factors(a, st, t);
     return;
   }
-  if (mode == 2 && mask_tile_skippable(a, blockIdx.x, blockIdx.y, gridDim.x, tiles_y)) return;
-  mask_tile<R, TH>(a, mode == 1, blockIdx.x, blockIdx.y, gridDim.x, mode == 2);
+  if (mode == 2 && mask_tile_skippable(a, blockIdx.x, ty, gridDim.x, tiles_y)) return;
+  mask_tile<R, TH>(a, mode == 1, blockIdx.x, ty, gridDim.x, mode == 2);
 }
 
 // check_solve of the N_RK = 2 step (mode 2) on a large domain: `group` tiles
@@ -2084,13 +2102,15 @@ template <class R, int NS, int TH, int ROWS, int MIN_BLOCKS>
 __global__ void __launch_bounds__(TX * ROWS, MIN_BLOCKS) k_stage2(KArgs<R> a, int mode) {
   step_kernel_entry();
   const bool go = a.st->run_step != 0;   // tested with the tile's code: one latency
-  const int kk = blockIdx.y * ROWS + threadIdx.x / TX;
+  const int by = stage_row<R>();
+  const int kk = by * ROWS + threadIdx.x / TX;
   // inactive, or left unchanged (k_flux's dry tiles, k_mask's dry border)
   auto skipped = [](uint8_t ta) { return ta == 0 || ta == 2 || ta == TILE_DRY_BORDER; };
   int tile;
   bool run = true;
   if constexpr (TH >= 8) {
-    tile = (blockIdx.y * ROWS / TH) * gridDim.x + blockIdx.x;
+    if (sizeof(R) == 8 && by * ROWS >= a.g.ny) return;
+    tile = (by * ROWS / TH) * gridDim.x + blockIdx.x;
     if (!go | skipped(a.tile_active[tile])) return;
   } else {
     // 32 x 4 tiles: the block's two halves belong to two tiles
@@ -2175,12 +2195,14 @@ __global__ void __launch_bounds__(StageShape<R>::THREADS, sizeof(R) == 4 ? 1 : 4
   constexpr int nv = 4 + NS;
   RunState* st = a.st;
   if (!st->run_step) return;
+  const int by = stage_row<R>();
   if constexpr (TH >= 8) {
-    if (!a.tile_active[(blockIdx.y * ROWS / TH) * gridDim.x + blockIdx.x]) return;
+    if (sizeof(R) == 8 && by * ROWS >= a.g.ny) return;
+    if (!a.tile_active[(by * ROWS / TH) * gridDim.x + blockIdx.x]) return;
   }
   const Grid<R>& g = a.g;
   const int j = blockIdx.x * TX + threadIdx.x % TX;
-  const int k = blockIdx.y * ROWS + threadIdx.x / TX;
+  const int k = by * ROWS + threadIdx.x / TX;
   unsigned status = 0;
   int nit = 0;
   if (j < g.nx && k < g.ny && (TH >= 8 || a.tile_active[(k / TH) * gridDim.x + blockIdx.x])) {
@@ -2224,12 +2246,14 @@ __global__ void __launch_bounds__(StageShape<R>::THREADS, sizeof(R) == 4 ? 1 : 4
   constexpr int nv = 4 + NS;
   RunState* st = a.st;
   if (!st->run_step) return;
+  const int by = stage_row<R>();
   if constexpr (TH >= 8) {
-    if (!a.tile_active[(blockIdx.y * ROWS / TH) * gridDim.x + blockIdx.x]) return;
+    if (sizeof(R) == 8 && by * ROWS >= a.g.ny) return;
+    if (!a.tile_active[(by * ROWS / TH) * gridDim.x + blockIdx.x]) return;
   }
   const Grid<R>& g = a.g;
   const int j = blockIdx.x * TX + threadIdx.x % TX;
-  const int k = blockIdx.y * ROWS + threadIdx.x / TX;
+  const int k = by * ROWS + threadIdx.x / TX;
   unsigned status = 0;
   if (j < g.nx && k < g.ny && (TH >= 8 || a.tile_active[(k / TH) * gridDim.x + blockIdx.x])) {
     const int64_t c = cidx(g, j, k);

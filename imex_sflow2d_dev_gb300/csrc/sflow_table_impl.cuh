@@ -130,7 +130,7 @@ static inline cudaError_t sm_count(int* sms) {
 // pointwise kernels of a single run: one block per 32 x ROWS cells
 template <class R>
 static inline dim3 stage_grid(dim3 tiles, int ny) {
-  return dim3(tiles.x, (unsigned)((ny + StageShape<R>::ROWS - 1) / StageShape<R>::ROWS));
+  return row_grid(tiles, (unsigned)((ny + StageShape<R>::ROWS - 1) / StageShape<R>::ROWS));
 }
 
 template <class R, int NS, int TH>
@@ -144,7 +144,7 @@ static cudaError_t tab_mask(const KArgs<R>& a, dim3 grid, cudaStream_t s, int so
   if (e != cudaSuccess) return e;
   const int group = mask_group(tiles, sms);
   if (group == 1 || solve_all != 2)
-    return launch_step_kernel(k_mask<R, TH>, dim3(grid.x, grid.y + src), T, 0, s, a.g.pdl, a, solve_all, ty);
+    return launch_step_kernel(k_mask<R, TH>, row_grid(grid, grid.y + src), T, 0, s, a.g.pdl, a, solve_all, ty);
   return launch_step_kernel(k_mask_group<R, TH>, dim3((unsigned)((tiles + group - 1) / group) + src), T, 0, s, a.g.pdl,
                             a, tx, ty, group);
 }
@@ -166,8 +166,8 @@ static cudaError_t tab_flux(const KArgs<R>& a, dim3 grid, size_t smem, cudaStrea
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
     const int sh = flux64_rows((int64_t)grid.x * grid.y, sms);
-    grid.y *= 8 / sh;
-    return launch_step_kernel(kern, grid, dim3(kFlux64Threads), smem, s, a.g.pdl, a, qin, rout, want_dt, sh);
+    return launch_step_kernel(kern, row_grid(grid, grid.y * (8 / sh)), dim3(kFlux64Threads), smem, s, a.g.pdl, a, qin,
+                              rout, want_dt, sh);
   } else {
     return launch_step_kernel(kern, grid, dim3(TileShape<TH>::FLUX_THREADS), smem, s, a.g.pdl, a, qin, rout, want_dt);
   }
