@@ -44,8 +44,9 @@ struct HostSetup {
   // topography (B_cent), row-major
   std::vector<double> B;
   // row slab of a larger domain (host_setup_rows): rows row0 .. row0+ny-1
-  // of it, of which own_lo .. own_hi-1 (local) are this domain's own
-  int row0 = 0, own_lo = 0, own_hi = 0;
+  // of it (ny_whole rows), of which own_lo .. own_hi-1 (local) are this
+  // domain's own
+  int row0 = 0, own_lo = 0, own_hi = 0, ny_whole = 0;
 };
 
 constexpr uint8_t kFlagNodata = 0x40;   // B_nodata cell

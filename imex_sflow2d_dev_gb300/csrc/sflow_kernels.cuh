@@ -47,10 +47,10 @@ constexpr int kTileHDefault = 8;
 
 // Thread blocks of a single run's pointwise kernels: 32 x ROWS cells, one
 // cell each, of one tile (or half a tile of 32 x 4).  k_stage2:
-//  FP32, SMALL (the blocks of 8 rows number at most 8 per SM): 4 rows, 12
-//        blocks per SM (40 registers); the kernel is one wave that waits on
-//        memory, and smaller blocks spread the wet ones over the SMs (640 x
-//        480 current with settling 25.0 -> 22.5 us against 8 rows, 6 blocks).
+//  FP32, SMALL (kStageSmallBlocks): 4 rows, 12 blocks per SM (40 registers);
+//        the kernel is one wave that waits on memory, and smaller blocks spread
+//        the wet ones over the SMs (640 x 480 current with settling 25.0 ->
+//        22.5 us against 8 rows, 6 blocks).
 //  FP32, else: 8 rows, 4 blocks per SM (64 registers, no spills): 4096^2
 //        current with settling and entrainment 575 -> 526 us, 1024^2 30.6 ->
 //        30.0 against 6 blocks per SM (40 registers); 5 blocks 533 and 30.7, 3
@@ -72,6 +72,20 @@ struct StageShape {
   static constexpr int SMALL_ROWS = sizeof(R) == 4 ? 4 : 2;
   static constexpr int SMALL_MIN_BLOCKS = sizeof(R) == 4 ? 12 : 4;
 };
+
+// SMALL: domains of at most so many blocks of 32 x 8 cells (eight per SM).
+// The two shapes differ in their FP32 results' last bits, so the line is a
+// number of its own, not one of the device, and a row slab goes by its whole
+// domain: it takes the shape that the undivided run takes.  Measured, 4 rows
+// against 8, us a launch, current with settling and entrainment in two
+// spreads (wet about a sixth and a third of the cells): 256 blocks 20.5 / 18.4
+// and 20.5 / 20.5, 650 20.5 / 20.5 and 24.5 / 24.6, 1,024 22.4 / 26.1 and 31.7
+// / 28.7, 1,064 22.2 / 25.8 and 26.6 / 28.7, 1,200 22.4 / 27.7 and 31.7 /
+// 28.7; 1,408 27.7 / 28.0 and 35.8 / 28.7, 1,900 33.5 / 28.7 and 38.9 / 30.5,
+// 4,096 42.1 / 39.1 and 68.0 / 63.3.  Without settling the two are within 2 us
+// of each other throughout.  (608 x 512, 1,216 blocks, 28.7 / 28.2 and 37.4 /
+// 28.7: probably since 19 columns of blocks put each column on 8 SMs of 152.)
+constexpr int64_t kStageSmallBlocks = 1216;
 
 // flag byte bits
 constexpr uint8_t F_SC_MASK = 0x3;  // source_cell (0, 1 ring interior, 2 ring boundary)

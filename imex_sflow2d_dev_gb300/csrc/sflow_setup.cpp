@@ -512,6 +512,7 @@ int host_setup(const SflowParams* pin, const double* B, HostSetup& s, std::strin
   ring_source(s);
   if (p.bottom_radial_source_flag) cell_fractions(s);
   s.row0 = 0;
+  s.ny_whole = s.ny;
   s.own_lo = 0;
   s.own_hi = s.ny;
   return SFLOW_OK;

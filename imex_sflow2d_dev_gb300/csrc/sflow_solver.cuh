@@ -1434,6 +1434,7 @@ class Solver : public SolverBase {
         ka_.bc.value[sd][i] = (R)p.bc[sd][i].value;
       }
     g.k_off = hs_.row0;
+    g.ny_whole = hs_.ny_whole;
     g.own_lo = hs_.own_lo;
     g.own_hi = hs_.own_hi;
     g.whole = (hs_.own_lo == 0 && hs_.own_hi == hs_.ny) ? 1 : 0;

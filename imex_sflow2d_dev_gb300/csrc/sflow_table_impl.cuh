@@ -185,10 +185,7 @@ static cudaError_t tab_stage2(const KArgs<R>& a, dim3 grid, cudaStream_t s, int 
     }
   }
   if constexpr (S::SMALL_ROWS != S::ROWS) {
-    int sms = 0;
-    const cudaError_t e = sm_count(&sms);
-    if (e != cudaSuccess) return e;
-    if ((int64_t)grid.x * ((a.g.ny + S::ROWS - 1) / S::ROWS) <= (int64_t)8 * sms)
+    if ((int64_t)grid.x * ((a.g.ny_whole + S::ROWS - 1) / S::ROWS) <= kStageSmallBlocks)
       return launch_step_kernel(k_stage2<R, NS, TH, S::SMALL_ROWS, S::SMALL_MIN_BLOCKS>,
                                 dim3(grid.x, (unsigned)((a.g.ny + S::SMALL_ROWS - 1) / S::SMALL_ROWS)),
                                 dim3(TX * S::SMALL_ROWS), 0, s, a.g.pdl, a, mode);

@@ -84,6 +84,7 @@ struct Grid {
   // counts, the status bits and the log sums take only rows own_lo .. own_hi-1
   int k_off, own_lo, own_hi;
   int whole;        // own_lo == 0 && own_hi == ny
+  int ny_whole;     // rows of the whole domain
 };
 
 // Device-resident run state (one per domain).
