@@ -388,7 +388,8 @@ int sflow_check_conversions(int64_t n, uint64_t seed, int64_t* mismatches) {
 }
 
 int sflow_eval_math(int32_t which, int64_t n, const double* x, const double* y, double* out) {
-  if (which < 0 || which > 5 || n < 0 || (n > 0 && (!x || !out)) || ((which == 0 || which == 3) && n > 0 && !y))
+  if (which < 0 || which > 7 || n < 0 || (n > 0 && (!x || !out)) ||
+      ((which == 0 || which == 3 || which == 6) && n > 0 && !y))
     return fail(SFLOW_EINVAL, "bad argument");
   const int rc = sflow::eval_math(which, (long long)n, x, y, out);
   if (rc != SFLOW_OK) return fail(rc, "device evaluation failed");

@@ -11,9 +11,10 @@ BatchBase* make_batch_fp64(int max_runs, int64_t max_tiles, std::string& err) {
   return make_batch_impl<double>(max_runs, max_tiles, err);
 }
 
-// The library's FP64 pow / log / cos (sflow_math.h, sflow_pow.h) evaluated on the device,
-// and CUDA's own functions beside them, for the test that compares the
-// device bits with the host bits of the same functions.
+// The library's FP64 pow / log / cos (sflow_math.h, sflow_pow.h), division and
+// square root (sflow_div64.cuh) evaluated on the device, and CUDA's own pow /
+// log / cos beside them, for the tests that compare the device bits with the
+// host bits of the same functions.
 __global__ void k_eval_math(int which, long long n, const double* x, const double* y, double* out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     double r;
@@ -23,6 +24,8 @@ __global__ void k_eval_math(int which, long long n, const double* x, const doubl
       case 2: r = sfm_cos(x[i]); break;
       case 3: r = pow(x[i], y[i]); break;
       case 4: r = log(x[i]); break;
+      case 6: r = ddiv64(x[i], y[i]); break;
+      case 7: r = dsqrt64(x[i]); break;
       default: r = cos(x[i]); break;
     }
     out[i] = r;

@@ -174,12 +174,12 @@ def check_conversions(n=1 << 22, seed=12345):
     return m.value
 
 
-MATH_FUNCS = {"pow": 0, "log": 1, "cos": 2, "cuda_pow": 3, "cuda_log": 4, "cuda_cos": 5}
+MATH_FUNCS = {"pow": 0, "log": 1, "cos": 2, "cuda_pow": 3, "cuda_log": 4, "cuda_cos": 5, "div": 6, "sqrt": 7}
 
 
 def eval_math(name, x, y=None):
-    """The library's FP64 pow / log / cos (or CUDA's, 'cuda_*') evaluated on
-    the device over the arrays x (and y for pow)."""
+    """The library's FP64 pow / log / cos / div / sqrt (or CUDA's, 'cuda_*')
+    evaluated on the device over the arrays x (and y for pow and div)."""
     lib = load()
     x = np.ascontiguousarray(x, dtype=np.float64).reshape(-1)
     out = np.empty_like(x)

@@ -310,8 +310,10 @@ int sflow_check_conversions(int64_t n, uint64_t seed, int64_t* mismatches);
 /* The FP64 pow (which 0), log (1) and cos (2) that the FP64 kernels use for
  * the settling, entrainment and inlet-ramp closures -- functions of this
  * library that give the same bits on the device as on the host -- and
- * CUDA's pow, log, cos (3, 4, 5), evaluated on the device for n host
- * arguments (y only for pow).  For tests of those functions. */
+ * CUDA's pow, log, cos (3, 4, 5); the correctly rounded quotient x / y (6)
+ * and square root (7) that they compute on the integer pipes; evaluated on
+ * the device for n host arguments (y only for pow and the quotient).  For
+ * tests of those functions. */
 int sflow_eval_math(int32_t which, int64_t n, const double* x, const double* y, double* out);
 
 #define SFLOW_TILE_CANDIDATES 3
