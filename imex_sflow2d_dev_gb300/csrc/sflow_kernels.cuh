@@ -1013,18 +1013,14 @@ __device__ __forceinline__ R kt_flux(const Side<R, NS>& L, const Side<R, NS>& Rt
   return rmax(a2, -a1);
 }
 
-// Both sides of a face of a special tile (domain edge, ring inlet or source
-// nearby): reconstruction, the domain-edge copies and the wall mirror at
-// ring-inlet faces (solver_2d.f90:3716-3920).  flags: bit 0 / 1 the low / high
-// side exists, bit 2 / 3 it is a wall mirror.
-template <class R, int NS>
-struct FaceStates {
-  R lo[4 + NS + 2], hi[4 + NS + 2];
-  int flags;
-};
+// The rules of a face in a special tile (domain edge, ring inlet or source
+// nearby) over the ordinary states of its two sides: the edge rules of a cell
+// at the domain edge or the ring, the domain-edge copies and the wall mirror
+// at ring-inlet faces (solver_2d.f90:3716-3920).  Returns bit 0 / 1: the low /
+// high side exists, bit 2 / 3: it is a wall mirror.
 template <class R, int NS, int DIR, int LIM, int TH>
-__device__ __forceinline__ FaceStates<R, NS> face_states_special(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f,
-                                                              int o, int rxl, int ryl, int rxh, int ryh) {
+__device__ __forceinline__ int face_special(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f, int o, int rxl,
+                                            int ryl, int rxh, int ryh, R* qpl, R* qph) {
   constexpr int nv = 4 + NS, np = nv + 2;
   constexpr int vel = (DIR == 1) ? nv : nv + 1;
   const int n = (DIR == 1) ? a.g.nx : a.g.ny;
@@ -1032,18 +1028,24 @@ __device__ __forceinline__ FaceStates<R, NS> face_states_special(const KArgs<R>&
   const uint8_t flh = (f < n) ? sfl[ryh * RX + rxh] : 0;
   const bool actl = fll & F_ACTIVE, acth = flh & F_ACTIVE;
   const bool radial = a.pr.radial_source;
-  const bool ring_l = radial && (fll & F_SC_MASK) == 2 && f - 1 > 0 && f - 1 < n - 1;
-  const bool ring_h = radial && (flh & F_SC_MASK) == 2 && f > 0 && f < n - 1;
+  const bool src_l = radial && (fll & F_SC_MASK) == 2, src_h = radial && (flh & F_SC_MASK) == 2;
+  const bool ring_l = src_l && f - 1 > 0 && f - 1 < n - 1;
+  const bool ring_h = src_h && f > 0 && f < n - 1;
   const bool mirror_h = actl && ring_l && ((DIR == 1) ? (fll & F_E) : ((fll & F_N) && !(fll & F_S)));
   const bool mirror_l = !mirror_h && acth && ring_h && ((DIR == 1) ? ((flh & F_W) && !(flh & F_E)) : (flh & F_S));
-  FaceStates<R, NS> s;
-  R* qpl = s.lo;
-  R* qph = s.hi;
-  bool hl = false, hh = false;
-  const int jl = (DIR == 1) ? f - 1 : o, kl = (DIR == 1) ? o : f - 1;
-  const int jh = (DIR == 1) ? f : o, kh = (DIR == 1) ? o : f;
-  if (f > 0 && actl) { recon_side<R, NS, DIR, LIM, TH>(a, sqp, sfl, rxl, ryl, jl, kl, 1, qpl); hl = true; }
-  if (f < n && acth && !mirror_h) { recon_side<R, NS, DIR, LIM, TH>(a, sqp, sfl, rxh, ryh, jh, kh, 0, qph); hh = true; }
+  bool hl = f > 0 && actl, hh = f < n && acth && !mirror_h;
+  if (hl && (f == 1 || f == n || src_l)) {
+    const QpSide<R, NS> s = recon_side_edge<R, NS, DIR, LIM, TH>(a, sqp, sfl, rxl, ryl, (DIR == 1) ? f - 1 : o,
+                                                                 (DIR == 1) ? o : f - 1, 1);
+#pragma unroll
+    for (int i = 0; i < np; ++i) qpl[i] = s.v[i];
+  }
+  if (hh && (f == 0 || f == n - 1 || src_h)) {
+    const QpSide<R, NS> s =
+        recon_side_edge<R, NS, DIR, LIM, TH>(a, sqp, sfl, rxh, ryh, (DIR == 1) ? f : o, (DIR == 1) ? o : f, 0);
+#pragma unroll
+    for (int i = 0; i < np; ++i) qph[i] = s.v[i];
+  }
   if (f == 0) {
 #pragma unroll
     for (int i = 0; i < np; ++i) qpl[i] = qph[i];
@@ -1066,7 +1068,21 @@ __device__ __forceinline__ FaceStates<R, NS> face_states_special(const KArgs<R>&
     qpl[vel] = -qpl[vel];
     hl = true;
   }
-  s.flags = (hl ? 1 : 0) | (hh ? 2 : 0) | (mirror_l ? 4 : 0) | (mirror_h ? 8 : 0);
+  return (hl ? 1 : 0) | (hh ? 2 : 0) | (mirror_l ? 4 : 0) | (mirror_h ? 8 : 0);
+}
+
+// The same out of line, by value (a pointer to the caller's arrays would keep
+// every face's states in local memory).
+template <class R, int NS>
+struct FaceStates {
+  R lo[4 + NS + 2], hi[4 + NS + 2];
+  int flags;
+};
+template <class R, int NS, int DIR, int LIM, int TH>
+__device__ __noinline__ FaceStates<R, NS> face_special_call(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, int f,
+                                                            int o, int rxl, int ryl, int rxh, int ryh,
+                                                            FaceStates<R, NS> s) {
+  s.flags = face_special<R, NS, DIR, LIM, TH>(a, sqp, sfl, f, o, rxl, ryl, rxh, ryh, s.lo, s.hi);
   return s;
 }
 
@@ -1076,40 +1092,48 @@ __device__ __forceinline__ FaceStates<R, NS> face_states_special(const KArgs<R>&
 // source cell in the tile's region, so both cells are ordinary.  (An inactive
 // cell holds no mass, and no neighbour of it does: its reconstructed state is
 // the dry one that an absent side has.)
-// The kernel is bound by instructions, two thirds of them not arithmetic; the
-// special faces' rules and their states in local memory were part of it for
-// every face.  With them on a path of their own, the cells' edge rules by value
-// out of line, and 4 blocks per SM (56 registers, a few spills; the
-// generic-limiter kernel is faster with its 72 registers and 3 blocks): k_flux
-// 47.4 -> 40.6 us on a 1024^2 current, 328 -> 264 on a 4096^2 one, k_b_flux 58
-// -> 48 on a batch of 64 floods.  A batch of 256 ring-inlet runs, most of whose
-// tiles are special: 99 -> 106 (111 with the whole special path out of line),
-// made up by check_solve; the same bits.
+// The kernel is bound by instructions, two thirds of them not arithmetic, so
+// every face takes the ordinary reconstruction, one copy of it, and the few
+// that have rules of their own take them afterwards.  With minmod these are out
+// of line, which leaves the registers (56 for 4 blocks per SM) to the others;
+// the generic-limiter kernel (more registers, fewer blocks) holds them inline
+// (517 x 333 collapse 17.8 us against 19.6 out of line).  Measured from the
+// kernel whose every face had the rules inline: k_flux 47.4 -> 40.5 us on a
+// 1024^2 current, 328 -> 263 on a 4096^2 one; k_b_flux 58 -> 47 on a batch of 64
+// floods, 99.8 -> 99.3 on a batch of 256 ring-inlet runs, most of whose tiles
+// are special (a copy of the reconstruction for plain tiles and one for special
+// faces: 106; tiles of 4 rows 116 before, 133 with two copies, 120 now); the same
+// bits.
 template <class R, int NS, int DIR, int LIM, int TH, bool FLUX>
 __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, bool plain, int f,
                                        int o, int rxl, int ryl, int rxh, int ryh, R gcs, R* H) {
   constexpr int np = 4 + NS + 2;
   R qpl[np], qph[np];
+  recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxl, ryl, f - 1, 1, qpl);
+  recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxh, ryh, f, 0, qph);
   int flags = 3;
-  // in a special tile the faces away from the edge and the ring are ordinary too
-  // (a batch of 256 ring-inlet runs, whose tiles are mostly special: 112.4 ->
-  // 111.3 us a launch)
-  const int n = (DIR == 1) ? a.g.nx : a.g.ny;
-  bool ordinary = plain;
-  if (!plain && f > 1 && f < n - 1) {
-    ordinary = !(a.pr.radial_source && ((sfl[ryl * RX + rxl] | sfl[ryh * RX + rxh]) & F_SC_MASK));
-  }
-  if (ordinary) {
-    recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxl, ryl, f - 1, 1, qpl);
-    recon_ordinary<R, NS, DIR, LIM, TH>(a, sqp, rxh, ryh, f, 0, qph);
-  } else {
-    const FaceStates<R, NS> s = face_states_special<R, NS, DIR, LIM, TH>(a, sqp, sfl, f, o, rxl, ryl, rxh, ryh);
+  if (!plain) {
+    // in a special tile most faces are ordinary too
+    const int n = (DIR == 1) ? a.g.nx : a.g.ny;
+    if (f <= 1 || f >= n - 1 || (a.pr.radial_source && ((sfl[ryl * RX + rxl] | sfl[ryh * RX + rxh]) & F_SC_MASK))) {
+      if constexpr (LIM == 1) {
+        FaceStates<R, NS> s;
 #pragma unroll
-    for (int i = 0; i < np; ++i) {
-      qpl[i] = s.lo[i];
-      qph[i] = s.hi[i];
+        for (int i = 0; i < np; ++i) {
+          s.lo[i] = qpl[i];
+          s.hi[i] = qph[i];
+        }
+        s = face_special_call<R, NS, DIR, LIM, TH>(a, sqp, sfl, f, o, rxl, ryl, rxh, ryh, s);
+#pragma unroll
+        for (int i = 0; i < np; ++i) {
+          qpl[i] = s.lo[i];
+          qph[i] = s.hi[i];
+        }
+        flags = s.flags;
+      } else {
+        flags = face_special<R, NS, DIR, LIM, TH>(a, sqp, sfl, f, o, rxl, ryl, rxh, ryh, qpl, qph);
+      }
     }
-    flags = s.flags;
   }
   Side<R, NS> L, Hs;
   if (flags & 1) side_from_qp<R, NS, DIR, FLUX>(a, qpl, gcs, L, flags & 4);
