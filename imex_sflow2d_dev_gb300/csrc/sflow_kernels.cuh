@@ -41,6 +41,15 @@ struct TileShape {
   static constexpr int FLUX_THREADS = (TX * (TH + 1) + 31) / 32 * 32;
   // resident blocks per SM the persistent flux kernel is compiled for
   static constexpr int FLUX_MIN_BLOCKS = (TH >= 16) ? 2 : (TH >= 8 ? 4 : 6);
+  // the same of the single-run kernel of limiters other than minmod everywhere.
+  // Left to itself it takes 78 to 93 registers: 2 blocks of 8 rows, 1 of 16.
+  // Two blocks of 16 (56 registers) restore what wet domains had before the
+  // special faces got a path of their own: 640 x 480 dam break, limiter 3, tiles
+  // of 16 rows 84 -> 62 us a step (66 then), 900 x 600 124 -> 91 (101).  Tiles of
+  // 8 rows stay unbounded: with 3 blocks that dam break took 63 instead of 76
+  // us, but consecutive wet tiles shared an SM where most are dry (517 x 333
+  // collapse 32.4 -> 33.4, 352 x 240 28.7 -> 30.6).  A tuned run has both.
+  static constexpr int FLUX_MIN_BLOCKS_GEN = (TH >= 16) ? 2 : 1;
   static constexpr int MASK_THREADS = TX * TH;
 };
 constexpr int kTileHDefault = 8;
@@ -1097,13 +1106,13 @@ __device__ __noinline__ FaceStates<R, NS> face_special_call(const KArgs<R>& a, c
 // that have rules of their own take them afterwards.  With minmod these are out
 // of line, which leaves the registers (56 for 4 blocks per SM) to the others;
 // the generic-limiter kernel (more registers, fewer blocks) holds them inline
-// (517 x 333 collapse 17.8 us against 19.6 out of line).  Measured from the
+// (batch of 128 ring-inlet runs, limiter 3, 94 us against 96 out of line).  Measured from the
 // kernel whose every face had the rules inline: k_flux 47.4 -> 40.5 us on a
 // 1024^2 current, 328 -> 263 on a 4096^2 one; k_b_flux 58 -> 47 on a batch of 64
 // floods, 99.8 -> 99.3 on a batch of 256 ring-inlet runs, most of whose tiles
 // are special (a copy of the reconstruction for plain tiles and one for special
-// faces: 106; tiles of 4 rows 116 before, 133 with two copies, 120 now); the same
-// bits.
+// faces: 106; tiles of 4 rows 116 before, 133 with two copies, 120 now); with
+// limiter 3, 128 such runs 111 -> 94 (167 with two copies); the same bits.
 template <class R, int NS, int DIR, int LIM, int TH, bool FLUX>
 __device__ __forceinline__ R face_flux(const KArgs<R>& a, const R* sqp, const uint8_t* sfl, bool plain, int f,
                                        int o, int rxl, int ryl, int rxh, int ryh, R gcs, R* H) {
@@ -1464,7 +1473,7 @@ static __global__ void k_dt(RunState* st, double max_dt) {
 }
 
 template <class R, int NS, int LIM, int TH, bool FLUX>
-__global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, LIM == 1 ? TileShape<TH>::FLUX_MIN_BLOCKS : 1)
+__global__ void __launch_bounds__(TileShape<TH>::FLUX_THREADS, LIM == 1 ? TileShape<TH>::FLUX_MIN_BLOCKS : TileShape<TH>::FLUX_MIN_BLOCKS_GEN)
     k_flux(KArgs<R> a, const R* __restrict__ qin, R* __restrict__ rout, int want_dt) {
   step_kernel_entry();
   const RunState* st = a.st;
