@@ -15,12 +15,16 @@
 //    more of the halo and the faces between blocks (per cell, 2.28, 2.53 and
 //    3.03 faces and 2.3, 3.4 and 5.6 closures of the halo), more rows leave
 //    SMs idle on small domains: flux64_rows picks;
-//  * 192 threads, 3 blocks per SM (112 registers, some spills): 18 warps cover
-//    the latency of the FP64 chains (512^2 current 224 us; 2 blocks without
-//    spills 288; 128 threads, 4 blocks 240).
+//  * 192 threads, 3 blocks per SM (96 registers, with spills): 18 warps cover
+//    the latency of the FP64 chains (512^2 current, 2 classes, 224 us; 2 blocks
+//    without spills 288; 128 threads, 4 blocks 240).  Shared memory is 59.7,
+//    68.4 and 77.1 KB a block with 1, 2 and 3 classes; three of the last do not
+//    fit an SM's 228 KB, so runs of 3 classes have 2 blocks and the spills all
+//    the same.
 // Measured, one kernel of the FP32 layout before -> after: 512^2 current
 // (96,000 wet cells) 346 -> 224 us, 200^2 dam break 164 -> 103, 64^2 102 -> 47,
-// eroding flood 184 -> 90, FP64 ensemble 328 -> 160 us per step.
+// eroding flood 184 -> 90, FP64 ensemble 328 -> 160 us per step.  (The 512^2
+// current with 1 and 3 classes: 189 and 282 us.)
 #pragma once
 #include "sflow_kernels.cuh"
 
